@@ -40,14 +40,16 @@ def _units(cuda: str):
                  "-I", INCLUDE, "-I", CSRC]
     common_cpp = ["g++", "-std=c++17", "-O2", "-fPIC", "-ffp-contract=off", "-Wall", "-Wno-unused-function",
                   "-I", INCLUDE, "-I", CSRC, "-I", os.path.join(cuda, "include")]
-    yield "render_f64.cu", common_cu + ["--fmad=false"]
+    # no contraction: the reference's rounding, and the strict FP64 orbits that rely on it
+    strict = common_cu + ["--fmad=false", "-DMBGB_STRICT_F64"]
+    yield "render_f64.cu", strict
     yield "render_f32.cu", common_cu
     yield "noalloc.cu", common_cu
-    yield "wave_f64.cu", common_cu + ["--fmad=false"]
+    yield "wave_f64.cu", strict
     yield "wave_f32.cu", common_cu
-    yield "wave_more_f64.cu", common_cu + ["--fmad=false"]
+    yield "wave_more_f64.cu", strict
     yield "wave_more_f32.cu", common_cu
-    yield "render_more_f64.cu", common_cu + ["--fmad=false"]
+    yield "render_more_f64.cu", strict
     yield "render_more_f32.cu", common_cu
     yield "post.cu", common_cu + ["--fmad=false"]
     yield "capi.cpp", common_cpp

@@ -292,6 +292,46 @@ static bool fast_mandelbulb(const mbgb_scene &s) {
          !s.ifsFoldingMode && !uses_primitives(s);
 }
 
+// The bounds of box_orbit_strict. round(round(sqrt(q))^2) and round(sqrt(q)) do not decrease
+// with q, so each test of the reference is one bound on q, found among the doubles next to the
+// tested value.
+static double first_square_from(const double value) {   // smallest q with fl(fl(sqrt q)^2) >= value
+  auto sq = [](double q) { const double r = sqrt(q); return r * r; };
+  double q = value;
+  while (sq(q) < value) q = nextafter(q, HUGE_VAL);
+  for (double d = nextafter(q, 0.0); sq(d) >= value; d = nextafter(q, 0.0)) q = d;
+  return q;
+}
+static double last_root_to(const double value) {   // largest q with fl(sqrt q) <= value
+  double q = value * value;
+  while (sqrt(q) > value) q = nextafter(q, 0.0);
+  for (double d = nextafter(q, HUGE_VAL); sqrt(d) <= value; d = nextafter(q, HUGE_VAL)) q = d;
+  return q;
+}
+template <typename T>
+static void fill_box_strict(const mbgb_scene &s, FractalT<T> &f) {
+  const double mR2 = s.mboxFoldingSphericalMin * s.mboxFoldingSphericalMin;
+  const double fR2 = s.mboxFoldingSphericalFixed * s.mboxFoldingSphericalFixed;
+  auto ordinary = [](double v) { return fabs(v) < 1e60; };
+  bool ok = s.formula == MBGB_FORMULA_TGLAD && !s.mboxRotationsEnabled && s.mboxMainRotZero && !s.tgladFoldingMode &&
+            !s.sphericalFoldingMode && s.mboxOffset[0] == 0.0 && s.mboxOffset[1] == 0.0 && s.mboxOffset[2] == 0.0 &&
+            s.mboxFoldingLimit >= 0.0 && ordinary(s.mboxFoldingLimit) && ordinary(s.mboxFoldingValue) &&
+            ordinary(s.mboxScale) && ordinary(s.constantFactor) && mR2 > 1e-60 && mR2 < 1e60 && fR2 > 1e-60 &&
+            fR2 < 1e60;
+  for (int c = 0; c < 3; c++) ok = ok && ordinary(s.julia[c]);
+  if (!ok) return;
+  const double k1 = fR2 / mR2;
+  int e;
+  f.boxStrict = 1;
+  f.boxQIn = (T)first_square_from(mR2);
+  f.boxQMid = (T)first_square_from(fR2);
+  f.boxQBail = (T)last_root_to(1024.0);
+  f.boxK1 = (T)k1;
+  f.boxK1Pow2 = k1 >= 1.0 && frexp(k1, &e) == 0.5;
+  const double fv = s.mboxFoldingValue;
+  if (fv > 1e-60 && frexp(fv, &e) == 0.5 && 2.0 * s.mboxFoldingLimit >= fv) f.boxFoldFar = (T)ldexp(fv, 50);
+}
+
 template <typename T>
 static void fill_fractal(const mbgb_scene &s, FractalT<T> &f) {
   memset(&f, 0, sizeof(f));
@@ -335,6 +375,7 @@ static void fill_fractal(const mbgb_scene &s, FractalT<T> &f) {
     f.leanSa = km1 > T(0) ? fR2 / km1 : T(0);
     f.leanSb = km1 > T(0) ? T(1) / km1 : T(0);
   }
+  if (sizeof(T) == 8) fill_box_strict(s, f);
   f.mbColX = (T)s.mboxColorFactorX;
   f.mbColY = (T)s.mboxColorFactorY;
   f.mbColZ = (T)s.mboxColorFactorZ;
@@ -870,6 +911,8 @@ static void clear_unused(FractalT<T> &f) {
     memset(f.mbRotZero, 0, sizeof(f.mbRotZero));
     f.mbScale = f.mbFoldLimit = f.mbFoldValue = f.mbMinR = f.mbFixedR = T(0);
     f.leanKm1 = f.leanSa = f.leanSb = T(0);
+    f.boxStrict = f.boxK1Pow2 = 0;
+    f.boxQIn = f.boxQMid = f.boxQBail = f.boxK1 = f.boxFoldFar = T(0);
     f.mbColX = f.mbColY = f.mbColZ = f.mbColR = f.mbColSp1 = f.mbColSp2 = T(0);
     for (int k = 0; k < 3; k++) f.mbOffset[k] = T(0);
     memset(f.mbMainRot, 0, sizeof(f.mbMainRot));

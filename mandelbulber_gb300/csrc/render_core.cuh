@@ -11,6 +11,7 @@
 #pragma once
 
 #include "lean_orbit.cuh"
+#include "lean_orbit64.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -252,6 +253,28 @@ __device__ __forceinline__ float mandelbox_fast(const FractalT<float> &f, const 
   return dist;
 }
 
+// Units built with --fmad=false (the FP64 policy's) round every operation of the reference;
+// only there is the strict orbit compute<double, 8, 0>'s twin.
+#ifdef MBGB_STRICT_F64
+constexpr bool kStrictF64 = true;
+#else
+constexpr bool kStrictF64 = false;
+#endif
+
+// The FP64 Mandelbox orbit (formula 8, normal mode) through box_orbit_strict.
+__device__ __forceinline__ double mandelbox_strict(const FractalT<double> &f, const V3<double> p, const int N,
+                                                   int &Lout, Counters &cnt, const double scale) {
+  const V3<double> c = f.juliaMode ? V3<double>{f.julia[0], f.julia[1], f.julia[2]}
+                                   : V3<double>{__dmul_rn(p.x, f.constantFactor), __dmul_rn(p.y, f.constantFactor),
+                                                __dmul_rn(p.z, f.constantFactor)};
+  int L;
+  const double dist = box_orbit_strict(f, p.x, p.y, p.z, c.x, c.y, c.z, N, L, scale);
+  cnt.orbit += (unsigned long long)(L + 1);
+  cnt.calls += 1;
+  Lout = L;
+  return dist;
+}
+
 // One Mandelbulb power-8 iteration (trig_optim, src/fractal.cpp:211-225) without
 // transcendentals: theta = asin(z/r) in [-pi/2, pi/2] has cos = rho/r >= 0 and sin = z/r;
 // phi = atan2(y, x) has cos = x/rho, sin = y/rho (phi = 0 when rho = 0, as atan2(0, 0)).
@@ -412,6 +435,10 @@ __device__ __forceinline__ T calc_distance(const FractalT<T> &f, const V3<T> poi
     } else {
       distance = compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
     }
+  } else if constexpr (kStrictF64 && sizeof(T) == 8 && FORMULA == 8) {
+    distance = f.boxStrict && box_strict_point(point.x, point.y, point.z)
+                   ? mandelbox_strict(f, point, N, Li, cnt, fparam)
+                   : compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
   } else {
     distance = compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
   }

@@ -838,7 +838,7 @@ __device__ __forceinline__ void volumetric_affine(const ParamsT<T> &p, const Ste
 // OVF (effects variant): the overflow pass's instantiation, whose fold of a long ray's records
 // traces the volumetric lights' shadows in line; the main pass's holds no fold.
 template <typename T, int FORMULA, bool FAST, bool EFX = false, bool OVF = false>
-__global__ void __launch_bounds__(128, (FAST && sizeof(T) == 4) ? 8 : 6) primary_kernel(const __grid_constant__ ParamsT<T> p, const __grid_constant__ FractalT<double> fd,
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : FAST ? 8 : 6) primary_kernel(const __grid_constant__ ParamsT<T> p, const __grid_constant__ FractalT<double> fd,
                                                       const FrameIO io, const WaveBufs<T> wb,
                                                       const FrameCam<T> *__restrict__ cams, const int ncams) {
   const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

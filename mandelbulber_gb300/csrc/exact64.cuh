@@ -175,17 +175,23 @@ __host__ __device__ __forceinline__ double mul_exact(const double a, const doubl
 }
 
 #ifdef __CUDACC__
-// a * b for any operands: the integer product where both the factor `a` and the product are
-// well inside the normal range (b in [2^-300, 2^300]), the FP64 pipe elsewhere (zeros, huge
-// values).
-__device__ __forceinline__ double mul_int(const double a, const double b) {
-  const uint32_t ea = (uint32_t)(f64_bits(a) >> 52) & 0x7ffu;
-  return ea - 600u <= 800u ? mul_exact(a, b) : __dmul_rn(a, b);
+// The same for any operands: the integer forms where both operands lie in [2^-423, 2^377], so
+// that every result is normal, the FP64 pipe elsewhere (zeros, huge and special values).
+__device__ __forceinline__ bool int_range(const double a) {
+  return ((uint32_t)(f64_bits(a) >> 52) & 0x7ffu) - 600u <= 800u;
 }
-// a * a.
+// a * b with b in [2^-300, 2^300]
+__device__ __forceinline__ double mul_int(const double a, const double b) {
+  return int_range(a) ? mul_exact(a, b) : __dmul_rn(a, b);
+}
 __device__ __forceinline__ double square_int(const double a) {
-  const uint32_t ea = (uint32_t)(f64_bits(a) >> 52) & 0x7ffu;
-  return ea - 600u <= 800u ? mul_exact(a, a) : __dmul_rn(a, a);
+  return int_range(a) ? mul_exact(a, a) : __dmul_rn(a, a);
+}
+__device__ __forceinline__ double div_int(const double n, const double d) {
+  return int_range(n) && int_range(d) ? div_exact(n, d) : __ddiv_rn(n, d);
+}
+__device__ __forceinline__ double sqrt_int(const double q) {   // q >= 0
+  return int_range(q) ? sqrt_exact(q) : __dsqrt_rn(q);
 }
 #endif
 

@@ -376,6 +376,12 @@ static void fill_fractal(const mbgb_scene &s, FractalT<T> &f) {
     f.leanSb = km1 > T(0) ? T(1) / km1 : T(0);
   }
   if (sizeof(T) == 8) fill_box_strict(s, f);
+  if (sizeof(T) == 8 && !s.analitycDE && s.formula >= 3 && s.formula <= 6 && !s.ifsFoldingMode &&
+      !s.tgladFoldingMode && !s.sphericalFoldingMode) {
+    static const double qEnd = last_root_to(1e10);
+    f.deltaStrict = 1;
+    f.deltaQEnd = (T)qEnd;
+  }
   f.mbColX = (T)s.mboxColorFactorX;
   f.mbColY = (T)s.mboxColorFactorY;
   f.mbColZ = (T)s.mboxColorFactorZ;

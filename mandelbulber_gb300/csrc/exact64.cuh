@@ -184,6 +184,14 @@ __device__ __forceinline__ bool int_range(const double a) {
 __device__ __forceinline__ double mul_int(const double a, const double b) {
   return int_range(a) ? mul_exact(a, b) : __dmul_rn(a, b);
 }
+// a * b for any two operands
+__device__ __forceinline__ double mul2_int(const double a, const double b) {
+  return int_range(a) && int_range(b) ? mul_exact(a, b) : __dmul_rn(a, b);
+}
+// 2 a
+__device__ __forceinline__ double twice_int(const double a) {
+  return int_range(a) ? bits_f64(f64_bits(a) + 0x10000000000000ull) : __dadd_rn(a, a);
+}
 __device__ __forceinline__ double square_int(const double a) {
   return int_range(a) ? mul_exact(a, a) : __dmul_rn(a, a);
 }

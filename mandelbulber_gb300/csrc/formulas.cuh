@@ -853,6 +853,129 @@ __device__ __forceinline__ T primitives(const FractalT<T> &f, const V3<T> point,
   return distance;
 }
 
+// The orbits of the finite-difference estimate for the quadratic formulas (3 fast_trig, 4
+// hypercomplex, 5 quaternion, 6 minus_fast_trig): `n` iterations of the point, or with `ends`
+// set, until r > 1e10. Returns r; L is the last iteration's index, n when none ended the orbit.
+// The values of compute_runtime<double, kModeDelta1 / kModeDelta2> bit for bit.
+//
+// What bounds it: GB300's FP64 pipe (exact64.cuh). compute_runtime takes ~33 instructions and a
+// root of 156 SM cycles per quaternion iteration; here the squares of the norm are the next
+// iteration's, r > 1e10 is a bound on r^2 compared as integers (the root is taken once, at the
+// end), products, quotients and roots are integer and leave 7 sums to the pipe. A quaternion's
+// fourth component is 0 from the start and stays so (an infinite x aside). One loop serves the four orbits of an
+// estimate in turn: unrolling them side by side overflows the instruction cache. An orbit that
+// turned NaN stays NaN in all four formulas, so it ends there (as one that never escaped) instead
+// of after n iterations of the pipe's slow special cases.
+template <int FORM>
+__device__ __forceinline__ double delta_orbit_strict(double x, double y, double z, const double cx, const double cy,
+                                                     const double cz, const int n, const bool ends,
+                                                     const uint64_t qEnd, int &L) {
+  double w = 0.0;
+  double xx = square_int(x), yy = square_int(y), zz = square_int(z), ww = 0.0;
+  double q = __dadd_rn(__dadd_rn(xx, yy), zz);
+  // a quaternion of infinite x has the fourth component 2 x 0 = NaN at the next iteration
+  auto infinite = [](const double v) { return (f64_bits(v) & 0x7fffffffffffffffull) == 0x7ff0000000000000ull; };
+  const double nan = bits_f64(0x7ff8000000000000ull);
+  L = 0;
+  if (FORM == 5 && n > 0 && infinite(x)) {
+    L = n;
+    q = nan;
+  }
+#pragma unroll 1
+  for (; L < n; L++) {
+    const double x2 = twice_int(x);
+    if (FORM == 3 || FORM == 6) {
+      const double s = __dadd_rn(xx, yy), temp = __dsub_rn(1.0, div_int(zz, s));
+      const double nx = mul2_int(__dsub_rn(xx, yy), temp), ny = mul2_int(mul2_int(x2, y), temp);
+      const double z2 = twice_int(z), nz = mul2_int(FORM == 3 ? -z2 : z2, sqrt_int(s));
+      x = __dadd_rn(nx, cx);
+      y = __dadd_rn(ny, cy);
+      z = __dadd_rn(nz, cz);
+    } else if (FORM == 5) {
+      const double nx = __dsub_rn(__dsub_rn(xx, yy), zz), ny = mul2_int(x2, y), nz = mul2_int(x2, z);
+      x = __dadd_rn(nx, cx);
+      y = __dadd_rn(ny, cy);
+      z = __dadd_rn(nz, cz);
+    } else {
+      const double y2 = twice_int(y), w2 = twice_int(w);
+      const double nx = __dsub_rn(__dsub_rn(__dsub_rn(xx, yy), zz), ww);
+      const double ny = __dsub_rn(mul2_int(x2, y), mul2_int(w2, z));
+      const double nz = __dsub_rn(mul2_int(x2, z), mul2_int(y2, w));
+      w = __dsub_rn(mul2_int(x2, w), mul2_int(y2, z));
+      x = __dadd_rn(nx, cx);
+      y = __dadd_rn(ny, cy);
+      z = __dadd_rn(nz, cz);
+      ww = square_int(w);
+    }
+    xx = square_int(x);
+    yy = square_int(y);
+    zz = square_int(z);
+    q = __dadd_rn(__dadd_rn(xx, yy), zz);
+    if (FORM == 4) q = __dadd_rn(q, ww);
+    const uint64_t qb = f64_bits(q) & 0x7fffffffffffffffull;
+    if (qb > qEnd) {
+      if (qb > 0x7ff0000000000000ull) {   // NaN
+        L = n;
+        break;
+      }
+      if (ends) break;
+      if (FORM == 5 && L + 1 < n && infinite(x)) {
+        L = n;
+        q = nan;
+        break;
+      }
+    }
+  }
+  return sqrt_int(q);
+}
+
+// r of the point's orbit and of its three neighbours at a step of 1e-10 (CalculateDistance's
+// delta-DE branch), each neighbour iterated as often as the point. Returns the point's last index.
+template <int FORM>
+__device__ __forceinline__ int delta_radii_strict(const FractalT<double> &f, const V3<double> &point, const int N,
+                                                  double r[4]) {
+  const double d = 1e-10;
+  double px = point.x, py = point.y, pz = point.z;
+  int n = N, last = 0;
+  double r0 = 0.0, r1 = 0.0, r2 = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < 4; k++) {
+    // (x + d) - d need not be x: the reference moves the point there and back
+    if (k == 1) {
+      px = __dadd_rn(px, d);
+    } else if (k == 2) {
+      px = __dsub_rn(px, d);
+      py = __dadd_rn(py, d);
+    } else if (k == 3) {
+      py = __dsub_rn(py, d);
+      pz = __dadd_rn(pz, d);
+    }
+    double cx = f.julia[0], cy = f.julia[1], cz = f.julia[2];
+    if (!f.juliaMode) {
+      cx = __dmul_rn(px, f.constantFactor);
+      cy = __dmul_rn(py, f.constantFactor);
+      cz = __dmul_rn(pz, f.constantFactor);
+    }
+    int L;
+    const double rk = delta_orbit_strict<FORM>(px, py, pz, cx, cy, cz, n, k == 0, f64_bits(f.deltaQEnd), L);
+    if (k == 0) {
+      last = L;
+      n = L < N ? L + 1 : N;
+      r0 = rk;
+    } else if (k == 1) {
+      r1 = rk;
+    } else if (k == 2) {
+      r2 = rk;
+    } else {
+      r[3] = rk;
+    }
+  }
+  r[0] = r0;
+  r[1] = r1;
+  r[2] = r2;
+  return last;
+}
+
 template <typename T>
 __device__ __noinline__ T calc_distance_runtime(const FractalT<T> *__restrict__ fp, V3<T> point, const T detailSize,
                                                const int N, const int minN, const bool normalMode, int *Lio,
@@ -899,30 +1022,56 @@ __device__ __noinline__ T calc_distance_runtime(const FractalT<T> *__restrict__ 
   } else {
     const T deltaDE = T(1e-10);
     int L;
-    const T r = compute_runtime<T, kModeDelta1>(fp, point, N, 0, &L, fparam);
-    *orbit += (unsigned long long)(L + 1);
-    const int retval = L;
-    *Lio = L;
-    point.x += deltaDE;
-    point.y += T(0);
-    point.z += T(0);
-    T r2 = compute_runtime<T, kModeDelta2>(fp, point, N, L, &L, fparam);
-    *orbit += (unsigned long long)(L + 1);
-    const T dr1 = m_fabs(r2 - r) / deltaDE;
-    point.x -= deltaDE;
-    point.y += deltaDE;
-    point.z += T(0);
-    r2 = compute_runtime<T, kModeDelta2>(fp, point, N, L, &L, fparam);
-    *orbit += (unsigned long long)(L + 1);
-    const T dr2 = m_fabs(r2 - r) / deltaDE;
-    point.x += T(0);
-    point.y -= deltaDE;
-    point.z += deltaDE;
-    r2 = compute_runtime<T, kModeDelta2>(fp, point, N, L, &L, fparam);
-    *orbit += (unsigned long long)(L + 1);
+    T r, dr1, dr2, dr3, dr;
+    int retval;
+    bool strict = false;
+    if constexpr (kStrictF64 && sizeof(T) == 8) strict = f.deltaStrict;
+    if (strict) {
+      if constexpr (kStrictF64 && sizeof(T) == 8) {
+        double rr[4];
+        if (f.formula == 5) L = delta_radii_strict<5>(f, point, N, rr);
+        else if (f.formula == 4) L = delta_radii_strict<4>(f, point, N, rr);
+        else if (f.formula == 3) L = delta_radii_strict<3>(f, point, N, rr);
+        else L = delta_radii_strict<6>(f, point, N, rr);
+        *orbit += 4 * (unsigned long long)(L + 1);
+        r = rr[0];
+        dr1 = div_int(m_fabs(rr[1] - r), deltaDE);
+        dr2 = div_int(m_fabs(rr[2] - r), deltaDE);
+        dr3 = div_int(m_fabs(rr[3] - r), deltaDE);
+        // the point that the differences leave behind (the primitives see it)
+        point.x = (point.x + deltaDE) - deltaDE;
+        point.y = (point.y + deltaDE) - deltaDE;
+        point.z += deltaDE;
+        dr = sqrt_int(dr1 * dr1 + dr2 * dr2 + dr3 * dr3);
+      }
+      retval = L;
+      *Lio = L;
+    } else {
+      r = compute_runtime<T, kModeDelta1>(fp, point, N, 0, &L, fparam);
+      *orbit += (unsigned long long)(L + 1);
+      retval = L;
+      *Lio = L;
+      point.x += deltaDE;
+      point.y += T(0);
+      point.z += T(0);
+      T r2 = compute_runtime<T, kModeDelta2>(fp, point, N, L, &L, fparam);
+      *orbit += (unsigned long long)(L + 1);
+      dr1 = m_fabs(r2 - r) / deltaDE;
+      point.x -= deltaDE;
+      point.y += deltaDE;
+      point.z += T(0);
+      r2 = compute_runtime<T, kModeDelta2>(fp, point, N, L, &L, fparam);
+      *orbit += (unsigned long long)(L + 1);
+      dr2 = m_fabs(r2 - r) / deltaDE;
+      point.x += T(0);
+      point.y -= deltaDE;
+      point.z += deltaDE;
+      r2 = compute_runtime<T, kModeDelta2>(fp, point, N, L, &L, fparam);
+      *orbit += (unsigned long long)(L + 1);
+      dr3 = m_fabs(r2 - r) / deltaDE;
+      dr = m_sqrt(dr1 * dr1 + dr2 * dr2 + dr3 * dr3);
+    }
     *calls += 4;
-    const T dr3 = m_fabs(r2 - r) / deltaDE;
-    const T dr = m_sqrt(dr1 * dr1 + dr2 * dr2 + dr3 * dr3);
     if (f.linearDE) distance = T(0.5) * r / dr;
     else distance = T(0.5) * r * m_log(r) / dr;
     if (distance < T(0)) distance = T(0);

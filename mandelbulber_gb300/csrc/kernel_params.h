@@ -77,6 +77,10 @@ struct FractalT {
   T mbRotInv[2][3][9];
   T amin, amax, bmin, bmax, cmin, cmax;
   T mbVaryFold, mbVaryMinR, mbVaryScaleVary, mbVaryWadd, mbVaryRPower;   // mandelboxVaryScale4D
+  // FP64 finite-difference estimate of a quadratic formula without pre-folds (delta_orbit_strict,
+  // formulas.cuh): whether it applies, and the largest |z|^2 whose rounded root is at most 1e10
+  int deltaStrict;
+  T deltaQEnd;
   // run-time formulas (formulas.cuh); each block is filled only when the formula (or a step
   // of the hybrid sequence) reads it, so frames that differ only in unused fields still share
   // a launch sequence

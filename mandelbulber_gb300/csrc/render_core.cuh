@@ -133,6 +133,20 @@ __host__ __device__ __forceinline__ T fparam_of(const FractalT<T> &f) {
 }  // namespace dev
 }  // namespace mbgb
 
+namespace mbgb {
+namespace dev {
+
+// Units built with --fmad=false (the FP64 policy's) round every operation of the reference;
+// only there are the strict orbits (lean_orbit64.cuh, delta_orbit_strict) the generic ones' twins.
+#ifdef MBGB_STRICT_F64
+constexpr bool kStrictF64 = true;
+#else
+constexpr bool kStrictF64 = false;
+#endif
+
+}  // namespace dev
+}  // namespace mbgb
+
 #include "formulas.cuh"
 
 namespace mbgb {
@@ -252,14 +266,6 @@ __device__ __forceinline__ float mandelbox_fast(const FractalT<float> &f, const 
   Lout = L;
   return dist;
 }
-
-// Units built with --fmad=false (the FP64 policy's) round every operation of the reference;
-// only there is the strict orbit compute<double, 8, 0>'s twin.
-#ifdef MBGB_STRICT_F64
-constexpr bool kStrictF64 = true;
-#else
-constexpr bool kStrictF64 = false;
-#endif
 
 // The FP64 Mandelbox orbit (formula 8, normal mode) through box_orbit_strict.
 __device__ __forceinline__ double mandelbox_strict(const FractalT<double> &f, const V3<double> p, const int N,

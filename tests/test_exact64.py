@@ -111,3 +111,29 @@ def test_strict_box_distance_equals_oracle(gpu_ctx, oracle, keys):
     np.testing.assert_array_equal(out.cpu().numpy(), ref)
     np.testing.assert_array_equal(it.cpu().numpy(), ref_it)
     np.testing.assert_array_equal(mi.cpu().numpy(), ref_mi)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("formula", [3, 4, 5, 6])
+@pytest.mark.parametrize("keys", [{}, {"linear_DE_mode": 1, "N": 3}, {"julia_mode": 1, "julia_a": -0.6, "julia_b": 0.3, "julia_c": 0.1},
+                                  {"fractal_constant_factor": 0.7, "N": 1}, {"minN": 5}], ids=str)
+def test_strict_finite_difference_equals_oracle(gpu_ctx, oracle, formula, keys):
+    # iterations equal and distances to log()'s last bits: the radii and their differences are
+    # the reference's doubles, and only the logarithm may round differently (2 ulp of 1e-16)
+    import torch
+    sc = W.workload("mandelbulb_640x480", 64, 48, formula=formula, analityc_DE_mode=0, **{"N": 60, **keys})
+    rng = np.random.default_rng(formula)
+    pts = rng.uniform(-1.6, 1.6, (3000, 3))
+    edge = [0.0, -0.0, 1.0, -1.0, 0.25, 1e-200, -1e-310, 3.0, -50.0, 1e9, 1e20, 1e160, np.inf, np.nan]
+    pts[:600] = rng.choice(edge, (600, 3))
+    det = np.full(len(pts), 1e-3)
+    ref, ref_it, ref_mi = oracle_lib.distance(oracle, sc, pts, det)
+    p, d = torch.tensor(pts, device="cuda"), torch.tensor(det, device="cuda")
+    out = torch.zeros(len(pts), dtype=torch.float64, device="cuda")
+    it = torch.zeros(len(pts), dtype=torch.int32, device="cuda")
+    mi = torch.zeros(len(pts), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    gpu_ctx.distance(sc, p.data_ptr(), d.data_ptr(), len(pts), out.data_ptr(), it.data_ptr(), mi.data_ptr(), mb.PREC_FP64)
+    np.testing.assert_array_equal(it.cpu().numpy(), ref_it)
+    np.testing.assert_array_equal(mi.cpu().numpy(), ref_mi)
+    np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=1e-15, atol=0.0, equal_nan=True)

@@ -1221,6 +1221,10 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
   wb.pool_cap = w.poolCap;
   wb.polish_all = o.polish_all;
   wb.refill_min = g.cfg.refill;
+  // a small FP32 stage over 16 warps per SM (its warps diverge less with fewer lanes: a 160x120
+  // Mandelbulb 246 -> 224 us), an FP64 one over one per sub-partition (the pipe's time does not
+  // depend on the lanes: a 64x48 FP64 Mandelbox 1.60 ms at 4 warps per SM, 1.69 at 16)
+  wb.spread = c->sms * (sizeof(T) == 4 ? 16 : 4);
   wb.orbit_refill = g.cfg.orbitRefill;
   wb.exact_hit = o.exact_hit ? 1 : 0;
   wb.npix = g.npix * rays;
@@ -1259,6 +1263,12 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
     occ1 = std::min(occ1, g.cfg.ctasPerSm);
     occ2 = std::min(occ2, g.cfg.ctasPerSm);
   }
+  // The FP64 Mandelbulb spends its time in asin, atan2, pow and sincos on the FP64 pipe, which
+  // one warp per SM sub-partition fills. More warps only share it, while fewer hold their lanes
+  // full from the job list and let the longest rays run alone: 192x192 deep zoom 231 -> 111 ms,
+  // 512x512 864 -> 829 ms at 1 CTA per SM (2: 126, 823; 3: 163, 841).
+  if (sizeof(T) == 8 && kf == 2 && g.cfg.ctasPerSm == 0) occ1 = occ2 = std::max(1, 128 / block);
+  wb.spread = std::min(wb.spread, c->sms * std::min(occ1, occ2) * (block / 32));
   L.grid = c->sms * occ1;
   L.grid2 = c->sms * occ2;
   L.block = block;

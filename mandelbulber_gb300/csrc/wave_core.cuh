@@ -313,6 +313,26 @@ __device__ __forceinline__ unsigned int claim_jobs(unsigned int *counter, const 
   return base + (unsigned int)__popc(mask & ((1u << lane) - 1u));
 }
 
+// How a stage's warps share its jobs. A stage with fewer jobs than lanes hands each warp only as
+// many as let `wb.spread` warps take part, and only the first warps take any (blocks start one
+// per SM, so those spread evenly over the SMs and their sub-partitions). `lanes`: the lanes of a
+// warp that take jobs; `warps`: the warps that do.
+struct JobShare {
+  unsigned int lanes, warps, refill;
+  bool idle;   // this lane takes none
+};
+template <typename T>
+__device__ __forceinline__ JobShare job_share(const WaveBufs<T> &wb, const unsigned int jobs) {
+  JobShare s;
+  const unsigned int spread = (unsigned int)wb.spread;
+  s.lanes = jobs >= 32u * spread ? 32u : max(1u, (jobs + spread - 1) / spread);
+  s.warps = (jobs + s.lanes - 1) / s.lanes;
+  s.refill = min((unsigned int)wb.refill_min, max(1u, s.lanes / 4));
+  const unsigned int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  s.idle = (threadIdx.x & 31u) >= s.lanes || warp >= s.warps;
+  return s;
+}
+
 // One pooled step record: dist, thr, step in a 16-byte (float) or 32-byte (double) slot.
 __device__ __forceinline__ void store_record(float *r, const float dist, const float thr, const float step,
                                              const float scan) {
@@ -859,7 +879,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : FAST ? 8 : 6) primar
   unsigned int *jobCounter = io.overflow_pass ? (wb.ctl + 4) : (wb.ctl + 0);
 
   // per-lane ray state
-  bool active = false, exhausted = false;
+  const JobShare share = job_share(wb, nJobs);
+  bool active = false, exhausted = share.idle;
   int64_t gp = 0;   // pixel of the batch
   int64_t ri = 0;   // ray: depth * npix_frame + gp
   int phase = 0, i = 0, buffCount = 0, iters = 0, bis = 0;
@@ -874,7 +895,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : FAST ? 8 : 6) primar
     // a warp claims new jobs once refill_min of its lanes are idle, or when none is busy
     const bool need = !active && !exhausted;
     const unsigned int needMask = __ballot_sync(0xffffffffu, need);
-    if (needMask && (__popc(needMask) >= (unsigned int)wb.refill_min || !__any_sync(0xffffffffu, active))) {
+    if (needMask && (__popc(needMask) >= share.refill || !__any_sync(0xffffffffu, active))) {
       if (io.budget_ns && (threadIdx.x & 31) == 0 && deadline_passed(io)) atomicExch(io.error_flag, 1);
       // the flag is only ever set by an expired deadline: no read (an L2 round trip) without one
       const bool stop = io.budget_ns && *(volatile int *)io.error_flag != 0;
@@ -2018,7 +2039,7 @@ __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const Fr
   Counters cnt{0, 0, 0, 0};
   LeanOrbit<FORMULA> orb(p.f);
   SecondaryRay<float> s{};
-  bool active = false, exhausted = false, orbiting = false;
+  bool active = false, exhausted = job_share(wb, njobs).idle, orbiting = false;
   float odist = 0.0f;
   for (;;) {
     // lanes whose orbit ended: the distance estimate's clamps, then the ray's step
@@ -2208,13 +2229,14 @@ __global__ void __launch_bounds__(128) secondary_kernel(const __grid_constant__ 
   const SecondaryJobs jn = secondary_jobs<T, EFX>(p, wb, nh);
   const unsigned int njobs = jn.nShadow + jn.nAO + jn.nAux + (unsigned int)wb.sample_nres * jn.nSamples;
   Counters cnt{0, 0, 0, 0};
-  bool active = false, exhausted = false;
+  const JobShare share = job_share(wb, njobs);
+  bool active = false, exhausted = share.idle;
   SecondaryRay<T> s{};
   for (;;) {
     // a warp claims new jobs once refill_min of its lanes are idle, or when none is busy
     const bool need = !active && !exhausted;
     const unsigned int needMask = __ballot_sync(0xffffffffu, need);
-    if (needMask && (__popc(needMask) >= (unsigned int)wb.refill_min || !__any_sync(0xffffffffu, active))) {
+    if (needMask && (__popc(needMask) >= share.refill || !__any_sync(0xffffffffu, active))) {
       if (io.budget_ns && (threadIdx.x & 31) == 0 && deadline_passed(io)) atomicExch(io.error_flag, 1);
       // the flag is only ever set by an expired deadline: no read (an L2 round trip) without one
       const bool stop = io.budget_ns && *(volatile int *)io.error_flag != 0;

@@ -30,7 +30,22 @@ constexpr double kPi = 3.14159265358979323846;
 __global__ void compile16_kernel(const float *__restrict__ image_float, int64_t n, double brightness,
                                  double contrast, int hdr, const int *__restrict__ gamma,
                                  uint16_t *__restrict__ image16) {
+  // brightness and contrast 1 without HDR change no value above 2^-29 (v - 0.5 + 0.5 is exact there,
+  // and smaller ones end as 0): the 24-bit product by 65535 is then one of integers
+  const bool plain = brightness == 1.0 && contrast == 1.0 && !hdr;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n; i += (int64_t)gridDim.x * blockDim.x) {
+    if (plain) {
+      const float u = image_float[i];
+      uint32_t r = 0;   // negative, NaN
+      if (u >= 1.0f) {
+        r = 65535u;
+      } else if (u > 2e-6f) {
+        const uint32_t b = __float_as_uint(u);
+        r = (uint32_t)(((uint64_t)((b & 0x7fffffu) | 0x800000u) * 65535u) >> (150u - (b >> 23)));
+      }
+      image16[i] = gamma ? (uint16_t)gamma[r] : (uint16_t)(r ? r - 1 : 0);
+      continue;
+    }
     float v = (float)((double)image_float[i] * brightness);
     v = (float)(((double)v - 0.5) * contrast + 0.5);
     if (v < 0.0f) v = 0.0f;
@@ -177,156 +192,329 @@ __global__ void ssao_kernel(const float *__restrict__ zbuf, const uint16_t *__re
   }
 }
 
+// Pairs of floats (value hi + lo, about 46 bits) for the horizon angles.
+struct F2 {
+  float h, l;
+};
+__device__ __forceinline__ F2 f2_quick(const float a, const float b) {   // |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return {s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ F2 f2_sum(const float a, const float b) {     // exact
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ F2 f2_add(const F2 a, const F2 b) {
+  const F2 s = f2_sum(a.h, b.h);
+  return f2_quick(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
+}
+__device__ __forceinline__ F2 f2_mul(const F2 a, const F2 b) {
+  const float p = __fmul_rn(a.h, b.h);
+  return f2_quick(p, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.h, -p))));
+}
+__device__ __forceinline__ F2 f2_of(const double v) {
+  const float h = (float)v;
+  return {h, (float)(v - (double)h)};
+}
+
 // One sample of the flat projection's horizon search (shared by every pixel): direction a,
-// radius r. A pixel at integer x samples column trunc(x + off): with off = k + f, k integer, the
-// rounded sum stays strictly between x + k and x + k + 1 for f in [1e-9, 1 - 1e-9] and is x + k
-// for f = 0, so the column is x + k and the bounds test one of integers; other offsets (`sure`
-// false: cos(pi / 2) = 6e-17 times a radius) are added in double.
-struct SsaoSample {
-  double offX, offY;    // r^2 scale cos, r^2 scale sin
-  int kx, ky;           // floor of the offsets
-  int maxX, maxY;       // largest column and row inside the picture: size - 2, size - 1 for f = 0
-  float cx, cy;         // the offsets in the projection plane at depth 1: off / w aspect persp
-  int sure;
+// radius r. A pixel at integer x samples column trunc(fl(x + off)). With off = k + f, k integer
+// and f in [1e-9, 1 - 1e-9], the rounded sum stays strictly between x + k and x + k + 1: column
+// x + k, inside the picture up to width - 2. Other offsets (cos(pi / 2) = 6e-17 times a radius) are
+// off = k + g, |g| < 1e-9, and the sum's rounding decides (near_column).
+struct __align__(16) SsaoSample {
+  float cx, cy;         // the offset in the projection plane at depth 1, off / w aspect persp
+  uint32_t cc;          // float |cx| + |cy| rounded up to a multiple of 4 units; its low bits: kNearX,
+                        // kNearY
+  int16_t kx, ky;       // k of the offset
+};
+constexpr uint32_t kNearX = 1, kNearY = 2;
+struct __align__(16) SsaoOffset {
+  double x, y;          // r^2 scale cos, r^2 scale sin
+  float cxl, cyl;       // what the floats cx, cy leave
+  float gx, gy;         // g of the offset, its magnitude rounded up
 };
 
-__global__ void ssao_table_kernel(SsaoSample *__restrict__ t, const int width, const int height, const double persp,
-                                  const int quality, const double *__restrict__ cs, const double *__restrict__ sn) {
+// Column (or row) of fl(b + g), b = x + k, |g| < 1e-9, and whether it lies in [0, last]: the sum
+// rounds to b where |g| is at most half the spacing of doubles on its side of b, 2^(e - 53) for b
+// in [2^e, 2^(e+1)) and half that below a power of two (ties go to b, whose last bit is 0). A
+// power of two compares with |g| as with |g| rounded up.
+__device__ __forceinline__ bool near_column(const int b, const float g, const int last, int &at) {
+  at = b;
+  if (b < 0 || b > last) return false;
+  if (g == 0.0f) return true;
+  if (b == 0) return g > 0.0f && last > 0;
+  const int e = 31 - __clz(b);
+  const float half = __uint_as_float((uint32_t)(127 + e - 53) << 23);
+  if (g < 0.0f) {
+    if (-g > ((b & (b - 1)) ? half : 0.5f * half)) at = b - 1;
+    return true;
+  }
+  return b < last || g <= half;
+}
+
+__global__ void ssao_table_kernel(SsaoSample *__restrict__ t, SsaoOffset *__restrict__ o, const int width,
+                                  const int height, const double persp, const int quality,
+                                  const double *__restrict__ cs, const double *__restrict__ sn) {
   const double w = (double)width, h = (double)height;
   const double scale = w / (double)(quality * quality) / 2.0, aspect = w / h;
   const int n = quality * (quality - 1);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int a = i / (quality - 1);
     const double r = (double)(i % (quality - 1) + 1), rr = r * r * scale;
-    SsaoSample s;
-    s.offX = rr * cs[a];
-    s.offY = rr * sn[a];
-    const double fx = floor(s.offX), fy = floor(s.offY), rx = s.offX - fx, ry = s.offY - fy;
-    s.kx = (int)fx;
-    s.ky = (int)fy;
-    s.maxX = width - (rx == 0.0 ? 1 : 2);
-    s.maxY = height - (ry == 0.0 ? 1 : 2);
-    s.cx = (float)(s.offX / w * aspect * persp);
-    s.cy = (float)(s.offY / h * persp);
-    s.sure = (rx == 0.0 || (rx >= 1e-9 && rx <= 1.0 - 1e-9)) && (ry == 0.0 || (ry >= 1e-9 && ry <= 1.0 - 1e-9));
-    t[i] = s;
+    const double x = rr * cs[a], y = rr * sn[a];
+    double kx = floor(x), ky = floor(y), gx = x - kx, gy = y - ky;
+    const F2 cx = f2_of(x / w * aspect * persp), cy = f2_of(y / h * persp);
+    uint32_t cc = (__float_as_uint(fabsf(cx.h) + fabsf(cy.h)) | 3u) + 1u;
+    auto near = [&](const double v, double &k, double &g, const uint32_t flag) {
+      if (g >= 1e-9 && g <= 1.0 - 1e-9) return;
+      cc |= flag;
+      k = rint(v);
+      g = v - k;   // exact: v is next to k
+    };
+    near(x, kx, gx, kNearX);
+    near(y, ky, gy, kNearY);
+    t[i] = SsaoSample{cx.h, cy.h, cc, (int16_t)kx, (int16_t)ky};
+    o[i] = SsaoOffset{x, y, cx.l, cy.l, (float)copysign((double)__double2float_ru(fabs(gx)), gx),
+                      (float)copysign((double)__double2float_ru(fabs(gy)), gy)};
   }
 }
 
-// ThreadSSAO for the flat projection, the values of ssao_kernel<double> bit for bit.
+// atan(k / 16), k = 0 .. 16, and pi / 2.
+__device__ const F2 kAtan16[17] = {
+    {0.0f, 0.0f}, {0.06241881102323532f, -1.0272779293885037e-09f}, {0.12435499578714371f, -1.240382241363136e-09f},
+    {0.18534794449806213f, 5.49763257140512e-09f}, {0.244978666305542f, -3.1786777654474463e-09f}, {0.30288487672805786f, -8.353086222712136e-09f},
+    {0.3587706685066223f, 1.7639498750554594e-09f}, {0.4124104380607605f, 3.5366267692182873e-09f}, {0.46364760398864746f, 5.01215868808913e-09f},
+    {0.5123894810676575f, -2.0756919738573743e-08f}, {0.5585992932319641f, 2.2111597886009804e-08f}, {0.6022873520851135f, -5.950149262190507e-09f},
+    {0.6435011029243469f, 5.868937336117597e-09f}, {0.6823165416717529f, 1.3202995141625706e-08f}, {0.7188299894332886f, 1.0188335508587443e-08f},
+    {0.7531512975692749f, -1.660708015549517e-08f}, {0.7853981852531433f, -2.1855694143368964e-08f}};
+constexpr F2 kHalfPi{1.5707963705062866f, -4.371138828673793e-08f};
+
+// atan(t / d) for d > 0, both in [1e-10, 1e10] or t = 0, to 4e-12: the ratio n / m <= 1 of the two
+// is turned by the nearest k / 16, s = (n - c m) / (m + c n) with |s| <= 1/32 + an ulp, and
+// atan(s) is its series to s^7.
+__device__ __forceinline__ F2 f2_atan(const F2 t, const F2 d) {
+  const bool neg = t.h < 0.0f;
+  const F2 u = neg ? F2{-t.h, -t.l} : t;
+  const bool swap = u.h > d.h;
+  const F2 n = swap ? d : u, m = swap ? u : d;
+  const int k = __float2int_rn(16.0f * __fdividef(n.h, m.h));
+  const float c = (float)k * 0.0625f;
+  const F2 num = f2_add(n, f2_mul(F2{-c, 0.0f}, m)), den = f2_add(m, f2_mul(F2{c, 0.0f}, n));
+  const float inv = __fdividef(1.0f, den.h), s0 = __fmul_rn(num.h, inv);
+  const float s1 = __fmul_rn(__fadd_rn(__fmaf_rn(-s0, den.h, num.h), __fmaf_rn(-s0, den.l, num.l)), inv);
+  const float ss = __fmul_rn(s0, s0);
+  const float series = __fmul_rn(__fmul_rn(s0, ss), __fmaf_rn(ss, __fmaf_rn(ss, -1.0f / 7.0f, 0.2f), -1.0f / 3.0f));
+  F2 r = f2_add(kAtan16[k], f2_add(F2{s0, s1}, F2{series, 0.0f}));
+  if (swap) r = f2_add(kHalfPi, F2{-r.h, -r.l});
+  return neg ? F2{-r.h, -r.l} : r;
+}
+
+// The flat horizon search's inputs and outputs. `open` receives the pixels that the FP32 pass
+// leaves to ssao_exact_kernel, `opens` their number.
+struct SsaoArgs {
+  const float *zbuf;
+  const uint16_t *opacity;
+  const uint8_t *colour;
+  uint16_t *image16;
+  int width, height, quality;
+  double persp, intensity;
+  const SsaoSample *samples;   // [quality][quality - 1]
+  const SsaoOffset *offsets;
+  uint32_t *opens;
+  uint32_t *open;
+};
+
+// Whether a sample of the pixel (x, y) lies inside the picture and off the pixel itself; its index.
+__device__ __forceinline__ bool ssao_sample(const SsaoArgs &g, const SsaoSample &s, const int i, const int x,
+                                            const int y, int &at) {
+  int xi = x + s.kx, yi = y + s.ky;
+  bool ok = xi >= 0 && xi <= g.width - 2 && yi >= 0 && yi <= g.height - 2;
+  if (s.cc & (kNearX | kNearY)) {   // the same for every pixel: uniform
+    const bool inX = (s.cc & kNearX) ? near_column(xi, g.offsets[i].gx, g.width - 1, xi) : xi >= 0 && xi <= g.width - 2;
+    const bool inY = (s.cc & kNearY) ? near_column(yi, g.offsets[i].gy, g.height - 1, yi) : yi >= 0 && yi <= g.height - 2;
+    ok = inX && inY;
+  }
+  ok = ok && !(xi == x && yi == y);
+  at = (ok ? yi : y) * g.width + (ok ? xi : x);
+  return ok;
+}
+
+// ThreadSSAO for the flat projection, the bytes of ssao_kernel<double>.
 //
-// What bounds it: the FP64 pipe (exact64.cuh). A sample's slope takes three quotients and a root
-// there, 870 SM cycles a warp, and of the quality - 1 samples of a direction only the steepest
-// counts. So a first pass brackets every slope in FP32, lo <= slope <= up, and keeps the largest
-// lo and the largest up of the other samples: where that lies below, one sample is the steepest
-// for certain and only it is computed in double (otherwise every sample whose bracket reaches the
-// largest lo). The brackets: with A(x) = (x / w - 1/2) aspect persp the plane distance is
-// dx = A(xx) dz + c z (c the offset's, dz the depth difference, exact in FP32 up to its
-// rounding), so FP32's error is below 2^-21 ((|A(x)| + |c|) |dz| + |c z|), far above the double
-// form's own; the root and quotients add 4e-6 relative. Columns and rows come from integers
-// (SsaoSample). What is left is mostly atan, once a direction.
-// 1920x1080, quality 20 (with the 16-bit step): 70.6 -> 5.65 ms.
-__global__ void __launch_bounds__(128) ssao_flat_kernel(
-    const float *__restrict__ zbuf, const uint16_t *__restrict__ opacity, const uint8_t *__restrict__ colour,
-    uint16_t *__restrict__ image16, const int width, const int height, const double persp, const int quality,
-    const double intensity, const SsaoSample *__restrict__ table) {
-  using mbgb::dev::div_int;
-  using mbgb::dev::sqrt_int;
-  const int64_t n = (int64_t)width * height;
-  const double w = (double)width, h = (double)height, aspect = w / h;
+// What bounds it: in double the FP64 pipe (exact64.cuh): a sample's slope takes three quotients
+// and a root there, 870 SM cycles a warp, a direction's atan 800. The output is 16 bits, so the
+// horizon angles are formed in FP32 with proven errors, and only a pixel whose error interval
+// holds a whole number is left to ssao_exact_kernel.
+//   * Per direction a first pass brackets every sample's slope, lo <= slope <= up, in plain FP32:
+//     with A(x) = (x / w - 1/2) aspect persp the plane distance is dx = A(xx) dz + c z (c the
+//     offset's, dz the depth difference), whose FP32 error is below
+//     e = 2^-21 ((|A(x)| + |c|) |dz| + |c z|); with y = 1 / distance the slope's relative error is
+//     e y and 4e-6 for the root and the products. Where the largest lo passes every other sample's
+//     up, that sample is the steepest for certain. Depths are scaled by 2^-20, which keeps the
+//     squares of the background's 1e20 finite and those of 1e-6 normal.
+//   * Its angle (or, where it is not certain, that of every sample whose bracket reaches the
+//     largest lo) is computed in pairs of floats: distance error 2^-21 e, atan to 4e-12. To
+//     these the double form's own rounding is added, 2^-49 of the plane positions.
+//   * Columns and rows come from integers and a sample is one 16-byte load (SsaoSample). (An
+//     instruction of the FP64 pipe costs its 20 cycles even with no lane active: the pass has none.)
+// What bounds it now is the first pass's issue rate, about 40 instructions a sample.
+// 1920x1080, quality 20, with the 16-bit step: every slope in double 70.6 ms, the steepest only
+// in double 5.65 ms, as it stands 2.41 ms.
+__global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ SsaoArgs g) {
+  const int64_t n = (int64_t)g.width * g.height;
+  const double w = (double)g.width, h = (double)g.height, aspect = w / h;
+  const int steps = g.quality - 1;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % width), y = (int)(i / width);
-    const float zf = zbuf[i];
-    const double z = (double)zf;
-    double total = 0.0;
-    if (z < 1e19) {
-      const double px = (div_int((double)x, w) - 0.5) * aspect, py = div_int((double)y, h) - 0.5;
-      const double x2 = px * z * persp, y2 = py * z * persp;
-      const float ax = (float)(px * persp), ay = (float)(py * persp);
-      // the depth of sample s, or false outside the picture and on the pixel itself
-      auto depth_at = [&](const SsaoSample &s, float &z2) {
-        int xi = x + s.kx, yi = y + s.ky;
-        if (s.sure) {
-          if (xi < 0 || xi > s.maxX || yi < 0 || yi > s.maxY) return false;
-        } else {
-          const double xx = (double)x + s.offX, yy = (double)y + s.offY;
-          if (xx < 0.0 || xx > (double)(width - 1) || yy < 0.0 || yy > (double)(height - 1)) return false;
-          xi = (int)xx;
-          yi = (int)yy;
-        }
-        if (xi == x && yi == y) return false;
-        z2 = zbuf[(int64_t)yi * width + xi];
-        return true;
-      };
+    const int x = (int)(i % g.width), y = (int)(i / g.width);
+    const float zf = g.zbuf[i];
+    double total = 0.0, error = 0.0;
+    if ((double)zf < 1e19) {
+      const F2 axp = f2_of((mbgb::dev::div_int((double)x, w) - 0.5) * aspect * g.persp);
+      const F2 ayp = f2_of((mbgb::dev::div_int((double)y, h) - 0.5) * g.persp);
+      const float aa = fabsf(axp.h) + fabsf(ayp.h);
+      bool open = !(zf > 1e-6f && zf < 1e6f && aa < 1e3f);   // outside the forms' range
+      const float zs = zf * 9.5367431640625e-07f;            // 2^-20
       auto bracket = [&](const SsaoSample &s, const float z2, float &lo, float &up) {
-        const float dz = z2 - zf, gx = ax + s.cx, gy = ay + s.cy, bx = s.cx * zf, by = s.cy * zf;
-        const float dx = fabsf(fmaf(gx, dz, bx)), dy = fabsf(fmaf(gy, dz, by));
-        const float e = 4.8e-7f * ((fabsf(ax) + fabsf(s.cx) + fabsf(ay) + fabsf(s.cy)) * fabsf(dz) + fabsf(bx) + fabsf(by));
-        const float m = fmaxf(dx, dy), q = __fdividef(fminf(dx, dy), m);
-        const float dr = m * sqrtf(fmaf(q, q, 1.0f));
-        const float drLo = fmaf(dr, 1.0f - 4e-6f, -e), drUp = fmaf(dr, 1.0f + 4e-6f, e);
-        if (!(m > 1e-25f) || !(drLo > 1e-25f)) {   // nothing certain
-          lo = -INFINITY;
-          up = INFINITY;
-          return;
-        }
-        const float near = __fdividef(-dz, drLo), wide = __fdividef(-dz, drUp);
-        lo = dz < 0.0f ? wide * (1.0f - 4e-6f) : near * (1.0f + 4e-6f);
-        up = dz < 0.0f ? near * (1.0f + 4e-6f) : wide * (1.0f - 4e-6f);
+        const float t = fmaf(-z2, 9.5367431640625e-07f, zs), cc = __uint_as_float(s.cc);
+        const float dx = fmaf(axp.h + s.cx, -t, s.cx * zs), dy = fmaf(ayp.h + s.cy, -t, s.cy * zs);
+        const float inv = rsqrtf(fmaf(dx, dx, dy * dy)), slope = t * inv;
+        const float e = fmaf(aa + cc, fabsf(t), cc * zs);
+        const float rel = fmaf(e, 4.8e-7f * inv, 4e-6f), d = 1.15f * fabsf(slope) * rel;
+        const bool known = rel < 0.1f && fabsf(slope) < 1e30f;   // (false for NaN)
+        lo = known ? slope - d : -INFINITY;
+        up = known ? slope + d : INFINITY;
       };
-      auto slope = [&](const SsaoSample &s, const float z2f) {
-        const double xx = (double)x + s.offX, yy = (double)y + s.offY, z2 = (double)z2f;
-        const double g = z2 * persp;
-        const double dx = (div_int(xx, w) - 0.5) * aspect * g - x2;
-        const double dy = (div_int(yy, h) - 0.5) * g - y2;
-        return div_int(-(z2 - z), sqrt_int(dx * dx + dy * dy));
+      // a sample's angle and the bound of its error
+      auto angle = [&](const SsaoSample &s, const int at, const float z2f, float &err) {
+        // the background's depth is 1e20: the slope does not change with the scale
+        const float scale = fabsf(z2f) > 1e6f ? 2.8421709430404007e-14f : 1.0f;   // 2^-45
+        const float z2 = z2f * scale, z1 = zf * scale, cc = __uint_as_float(s.cc);
+        const F2 dz = f2_sum(z2, -z1), z{z1, 0.0f}, cx{s.cx, g.offsets[at].cxl}, cy{s.cy, g.offsets[at].cyl};
+        const F2 dx = f2_add(f2_mul(f2_add(axp, cx), dz), f2_mul(cx, z));
+        const F2 dy = f2_add(f2_mul(f2_add(ayp, cy), dz), f2_mul(cy, z));
+        const F2 q = f2_add(f2_mul(dx, dx), f2_mul(dy, dy));
+        const float inv = rsqrtf(q.h), r0 = __fmul_rn(q.h, inv);
+        const F2 dr = f2_quick(r0, __fmul_rn(__fmul_rn(0.5f, inv), __fadd_rn(__fmaf_rn(-r0, r0, q.h), q.l)));
+        if (!(dr.h > 1e-10f && fabsf(dz.h) < 1e7f)) open = true;
+        const float e = 4.8e-7f * fmaf(aa + cc, fabsf(dz.h), cc * z1);
+        err = 4e-12f + __fdividef(fmaf(e, 4.8e-7f, 1.8e-15f * (aa + cc) * (z1 + fabsf(z2))), dr.h);
+        return f2_atan(F2{-dz.h, -dz.l}, dr);
       };
-      double ambient = 0.0;
-      for (int a = 0; a < quality; a++) {
-        const SsaoSample *dir = table + (int64_t)a * (quality - 1);
+      F2 sum{0.0f, 0.0f};
+      float errSum = 0.0f;
+      for (int a = 0; a < g.quality; a++) {
+        const int first = a * steps;
         float bestLo = -INFINITY, bestUp = -INFINITY, otherUp = -INFINITY;
         int best = -1;
-        for (int r = 0; r < quality - 1; r++) {
-          float z2, lo, up;
-          if (!depth_at(dir[r], z2)) continue;
-          bracket(dir[r], z2, lo, up);
-          if (lo > bestLo || best < 0) {
-            otherUp = fmaxf(otherUp, bestUp);
-            bestLo = lo;
-            bestUp = up;
-            best = r;
-          } else {
-            otherUp = fmaxf(otherUp, up);
+#pragma unroll 4
+        for (int r = 0; r < steps; r++) {
+          const SsaoSample s = g.samples[first + r];
+          int at;
+          const bool ok = ssao_sample(g, s, first + r, x, y, at);
+          float lo, up;
+          bracket(s, g.zbuf[at], lo, up);
+          lo = ok ? lo : -INFINITY;
+          up = ok ? up : -INFINITY;
+          const bool better = lo > bestLo;
+          otherUp = fmaxf(otherUp, better ? bestUp : up);
+          bestLo = better ? lo : bestLo;
+          bestUp = better ? up : bestUp;
+          best = better ? r : best;
+        }
+        F2 top{-kHalfPi.h, -kHalfPi.l};   // no sample: the slope -1e50
+        float err = 0.0f;
+        int at;
+        if (best >= 0 && otherUp < bestLo) {
+          const SsaoSample s = g.samples[first + best];
+          ssao_sample(g, s, first + best, x, y, at);
+          top = angle(s, first + best, g.zbuf[at], err);
+        } else if (otherUp > -INFINITY) {
+          for (int r = 0; r < steps; r++) {
+            const SsaoSample s = g.samples[first + r];
+            if (!ssao_sample(g, s, first + r, x, y, at)) continue;
+            const float z2 = g.zbuf[at];
+            float lo, up, er;
+            bracket(s, z2, lo, up);
+            if (!(up >= bestLo)) continue;
+            const F2 t = angle(s, first + r, z2, er);
+            err = fmaxf(err, er);
+            if (t.h > top.h || (t.h == top.h && t.l > top.l)) top = t;
           }
         }
-        double maxDiff = -1e50;
-        if (best >= 0) {
-          if (otherUp < bestLo) {
-            float z2;
-            depth_at(dir[best], z2);
-            const double diff = slope(dir[best], z2);
-            if (diff > maxDiff) maxDiff = diff;
-          } else {
-            for (int r = 0; r < quality - 1; r++) {
-              float z2, lo, up;
-              if (!depth_at(dir[r], z2)) continue;
-              bracket(dir[r], z2, lo, up);
-              if (!(up >= bestLo)) continue;
-              const double diff = slope(dir[r], z2);
-              if (diff > maxDiff) maxDiff = diff;
-            }
-          }
-        }
-        ambient += div_int(-atan(maxDiff), kPi) + 0.5;
+        sum = f2_add(sum, top);
+        errSum += err;
       }
-      total = ambient / (double)quality;
-      if (total < 0.0) total = 0.0;
+      // the mean of 1/2 - angle / pi, and its error with that of the summation
+      const double per = 1.0 / (kPi * g.quality);
+      total = 0.5 - ((double)sum.h + (double)sum.l) * per;
+      error = ((double)errSum * 1.001 + 1e-12 * g.quality) * per;
+      if (open || !(error < 1e-3)) error = 2.0;
     }
-    const double op = (double)opacity[i] / 65535.0;
+    const double op = (double)g.opacity[i] / 65535.0;
+    const double gain = 65535.0 / 256.0 * g.intensity * (1.0 - op);
+    const double lowT = fmax(total - error, 0.0), highT = fmax(total + error, 0.0);
+    // (an error of 0 is the background's: its term is exactly 0)
+    bool settled = error == 0.0 || (error < 1.0 && g.intensity >= 0.0);
+    uint16_t out[3];
     for (int c = 0; c < 3; c++) {
-      double v = (double)image16[3 * i + c] + 65535.0 * (double)colour[3 * i + c] / 256.0 * total * intensity * (1.0 - op);
+      const uint16_t was = g.image16[3 * i + c];
+      const double base = (double)was, k = error == 0.0 ? 0.0 : gain * (double)g.colour[3 * i + c];
+      const double lo = fmin(base + k * lowT - 1e-9, 65535.0), hi = fmin(base + k * highT + 1e-9, 65535.0);
+      out[c] = k > 0.0 ? (uint16_t)(unsigned short)hi : was;
+      if (k > 0.0 && (uint16_t)(unsigned short)fmax(lo, 0.0) != out[c]) settled = false;
+    }
+    if (settled) {
+      for (int c = 0; c < 3; c++) g.image16[3 * i + c] = out[c];
+    } else {
+      g.open[atomicAdd(g.opens, 1u)] = (uint32_t)i;
+    }
+  }
+}
+
+// The pixels that ssao_flat_kernel leaves open, every slope in double as ThreadSSAO forms it (the
+// values of ssao_kernel<double> bit for bit), one warp a pixel: a lane takes every 32nd direction,
+// and the directions' terms are summed in the reference's order.
+__global__ void __launch_bounds__(128) ssao_exact_kernel(const __grid_constant__ SsaoArgs g) {
+  using mbgb::dev::div_int;
+  using mbgb::dev::sqrt_int;
+  const uint32_t n = *g.opens;
+  const double w = (double)g.width, h = (double)g.height, aspect = w / h;
+  const int lane = threadIdx.x & 31, steps = g.quality - 1;
+  for (uint32_t k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < n; k += gridDim.x * (blockDim.x >> 5)) {
+    const int64_t i = g.open[k];
+    const int x = (int)(i % g.width), y = (int)(i / g.width);
+    const double z = (double)g.zbuf[i];
+    double ambient = 0.0;
+    const double x2 = (div_int((double)x, w) - 0.5) * aspect * z * g.persp;
+    const double y2 = (div_int((double)y, h) - 0.5) * z * g.persp;
+    for (int a0 = 0; a0 < g.quality; a0 += 32) {
+      double term = 0.0;
+      if (a0 + lane < g.quality) {
+        const int first = (a0 + lane) * steps;
+        double maxDiff = -1e50;
+        for (int r = 0; r < steps; r++) {
+          int at;
+          if (!ssao_sample(g, g.samples[first + r], first + r, x, y, at)) continue;
+          const double xx = (double)x + g.offsets[first + r].x, yy = (double)y + g.offsets[first + r].y;
+          const double z2 = (double)g.zbuf[at], q = z2 * g.persp;
+          const double dx = (div_int(xx, w) - 0.5) * aspect * q - x2;
+          const double dy = (div_int(yy, h) - 0.5) * q - y2;
+          const double diff = div_int(-(z2 - z), sqrt_int(dx * dx + dy * dy));
+          if (diff > maxDiff) maxDiff = diff;
+        }
+        term = div_int(-atan(maxDiff), kPi) + 0.5;
+      }
+      for (int l = 0; l < 32 && a0 + l < g.quality; l++) ambient += __shfl_sync(0xffffffffu, term, l);
+    }
+    double total = ambient / (double)g.quality;
+    if (total < 0.0) total = 0.0;
+    if (lane < 3) {
+      const double op = (double)g.opacity[i] / 65535.0;
+      double v = (double)g.image16[3 * i + lane] +
+                 65535.0 * (double)g.colour[3 * i + lane] / 256.0 * total * g.intensity * (1.0 - op);
       if (v > 65535.0) v = 65535.0;
-      image16[3 * i + c] = (uint16_t)(unsigned short)v;
+      g.image16[3 * i + lane] = (uint16_t)(unsigned short)v;
     }
   }
 }
@@ -364,16 +552,32 @@ mbgb_status compile16_device(const mbgb_scene &scene, const float *image_float, 
   return MBGB_OK;
 }
 
-size_t ssao_scratch_bytes(int quality) {
-  const size_t q = (size_t)std::max(quality, 0);
-  return sizeof(double) * 2 * q + (q > 0 ? sizeof(SsaoSample) * q * (q - 1) : 0) + 64;
+// Scratch of ssao_device: cos and sin of the directions, their samples, the open pixels.
+struct SsaoScratch {
+  SsaoSample *samples;
+  SsaoOffset *offsets;
+  uint32_t *opens, *open;
+  size_t bytes;
+};
+static SsaoScratch ssao_scratch(void *base, int quality, int64_t npix) {
+  const size_t q = (size_t)std::max(quality, 0), n = q > 0 ? q * (q - 1) : 0;
+  size_t at = (sizeof(double) * 2 * q + 15) & ~(size_t)15;
+  SsaoScratch m;
+  m.samples = (SsaoSample *)((char *)base + at);
+  at += sizeof(SsaoSample) * n;
+  m.offsets = (SsaoOffset *)((char *)base + at);
+  at += sizeof(SsaoOffset) * n;
+  m.opens = (uint32_t *)((char *)base + at);
+  m.open = m.opens + 4;
+  m.bytes = at + 16 + sizeof(uint32_t) * (size_t)npix;
+  return m;
 }
+size_t ssao_scratch_bytes(int quality, int64_t npix) { return ssao_scratch(nullptr, quality, npix).bytes; }
 
 // PostRendering_SSAO on the device, in double (the reference's arithmetic): the sample
 // positions x + r^2 s cos(a) land on the neighbouring pixel or not depending on the last
 // bits of cos(a) near 0 (cos(pi / 2) = 6e-17), which float arithmetic does not keep.
-// `tables` (ssao_scratch_bytes) receives cos and sin of the `quality` directions and, for the
-// flat projection, the directions' samples.
+// `tables`: device scratch of ssao_scratch_bytes.
 mbgb_status ssao_device(const mbgb_scene &scene, const mbgb_image &layers, uint16_t *image16, void *tables,
                         cudaStream_t s) {
   const int q = scene.SSAOQuality;
@@ -388,17 +592,21 @@ mbgb_status ssao_device(const mbgb_scene &scene, const mbgb_image &layers, uint1
   const double *cs = (const double *)tables, *sn = cs + q;
   cudaError_t e = cudaMemcpyAsync(tables, t.data(), sizeof(double) * 2 * q, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) {
-    if (scene.perspectiveType == MBGB_PERSP_FISH_EYE || scene.perspectiveType == MBGB_PERSP_EQUIRECT) {
+    // (offsets past 16 bits and pixel indices past 31 take the general kernel too)
+    if (scene.perspectiveType == MBGB_PERSP_FISH_EYE || scene.perspectiveType == MBGB_PERSP_EQUIRECT ||
+        layers.width > 64000 || n >= (int64_t)1 << 31) {
       ssao_kernel<double><<<grid_for(n, block), block, 0, s>>>(
           layers.zbuffer, layers.opacity, layers.colour, image16, layers.width, layers.height, scene.persp, q,
           scene.perspectiveType, scene.globalIlum, cs, sn);
     } else {
-      SsaoSample *table = (SsaoSample *)(cs + 2 * q);
-      ssao_table_kernel<<<grid_for((int64_t)q * (q - 1), block), block, 0, s>>>(table, layers.width, layers.height,
-                                                                                scene.persp, q, cs, sn);
-      ssao_flat_kernel<<<grid_for(n, block), block, 0, s>>>(layers.zbuffer, layers.opacity, layers.colour, image16,
-                                                            layers.width, layers.height, scene.persp, q,
-                                                            scene.globalIlum, table);
+      const SsaoScratch m = ssao_scratch(tables, q, n);
+      const SsaoArgs g{layers.zbuffer, layers.opacity, layers.colour, image16, layers.width, layers.height, q,
+                       scene.persp, scene.globalIlum, m.samples, m.offsets, m.opens, m.open};
+      e = cudaMemsetAsync(m.opens, 0, sizeof(uint32_t), s);
+      ssao_table_kernel<<<grid_for((int64_t)q * (q - 1), block), block, 0, s>>>(m.samples, m.offsets, layers.width,
+                                                                                layers.height, scene.persp, q, cs, sn);
+      ssao_flat_kernel<<<grid_for(n, block), block, 0, s>>>(g);
+      ssao_exact_kernel<<<grid_for(n, block), block, 0, s>>>(g);
     }
   }
   if (e == cudaSuccess) e = cudaGetLastError();

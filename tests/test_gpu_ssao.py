@@ -32,7 +32,7 @@ def _depth(kind, w, h, rng):
     return 5.0 + np.sin(x * 0.3) + np.cos(y * 0.2) + 0.05 * rng.normal(size=(h, w))
 
 
-@pytest.mark.parametrize("w,h,quality", [(33, 32, 1), (64, 48, 2), (97, 55, 5), (131, 67, 20), (48, 200, 33)])
+@pytest.mark.parametrize("w,h,quality", [(33, 32, 1), (1, 40, 7), (64, 48, 2), (97, 55, 5), (131, 67, 20), (48, 200, 33)])
 @pytest.mark.parametrize("kind", ["plane", "flat", "steps", "tiny", "waves"])
 def test_flat_ssao_equals_oracle(gpu_ctx, oracle, w, h, quality, kind):
     import torch

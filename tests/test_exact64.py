@@ -86,20 +86,23 @@ BOXES = [{}, {"mandelbox_scale": -1.5}, {"mandelbox_scale": -2.0}, {"mandelbox_s
          {"mandelbox_folding_limit": 0.6, "mandelbox_folding_value": 2.0},
          {"mandelbox_folding_value": -2.0}, {"mandelbox_folding_limit": 0.0},
          {"julia_mode": 1, "julia_a": 0.3, "julia_b": -0.7, "julia_c": 0.0}, {"fractal_constant_factor": 0.5},
-         {"N": 1}, {"N": 250}]
+         {"N": 1}, {"N": 250}, {"interior_mode": 1}, {"iteration_threshold_mode": 1},
+         {"limits_enabled": 1, "x_min": -3, "x_max": 2.5, "y_min": -4, "y_max": 1, "z_min": -5, "z_max": 5}]
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 4133])
 @pytest.mark.parametrize("keys", BOXES, ids=[",".join(f"{k.split('_')[-1]}={v}" for k, v in b.items()) or "usual" for b in BOXES])
-def test_strict_box_distance_equals_oracle(gpu_ctx, oracle, keys):
+def test_strict_box_distance_equals_oracle(gpu_ctx, oracle, keys, n):
     import torch
     sc = W.workload("mandelbox_1080p", 64, 48, **keys)
     rng = np.random.default_rng(11)
-    pts = rng.uniform(-6.5, 6.5, (4096, 3))
+    pts = rng.uniform(-6.5, 6.5, (4133, 3))
     pts[:64] *= 0.05
     edge = [0.0, -0.0, 1.0, -1.0, 0.5, 2.0, 3.0, 1e-200, -1e-310, 0.25, 1e15, -4e15, 1e30, 1e95, 1e200, -1e300, np.inf,
             np.nan]
     pts[64:64 + 2000] = rng.choice(edge, (2000, 3))
+    pts = np.ascontiguousarray(pts[:n])
     det = np.full(len(pts), 1e-3)
     ref, ref_it, ref_mi = oracle_lib.distance(oracle, sc, pts, det)
     p, d = torch.tensor(pts, device="cuda"), torch.tensor(det, device="cuda")
@@ -109,7 +112,8 @@ def test_strict_box_distance_equals_oracle(gpu_ctx, oracle, keys):
     torch.cuda.synchronize()
     gpu_ctx.distance(sc, p.data_ptr(), d.data_ptr(), len(pts), out.data_ptr(), it.data_ptr(), mi.data_ptr(), mb.PREC_FP64)
     np.testing.assert_array_equal(out.cpu().numpy(), ref)
-    np.testing.assert_array_equal(it.cpu().numpy(), ref_it)
+    # beyond the limit box no orbit runs: itersOut stays as it was (the oracle's -1, the kernel's 0)
+    np.testing.assert_array_equal(it.cpu().numpy(), np.where(ref_it == -1, 0, ref_it))
     np.testing.assert_array_equal(mi.cpu().numpy(), ref_mi)
 
 

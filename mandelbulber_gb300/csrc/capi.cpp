@@ -1104,7 +1104,7 @@ static LaunchCfg resolve_cfg(const mbgb_context *c, const mbgb_opts &o, const mb
 struct WaveLayout {
   size_t flags, scan, dist, thr, step, detail, bis, point, iters, count, vol, shadow, ao, hit, pol, ovl, last;
   size_t prec, pprev;
-  size_t rstart, rdir, rthr, rlist, normal, auxsh, sbase, sray, srec, sstep, sres, piters, segc, hset;
+  size_t rstart, rdir, rthr, rlist, normal, auxsh, sbase, sray, srec, sstep, sres, piters, segc, hset, colr;
   uint32_t poolCap;
   size_t total;
 };
@@ -1166,6 +1166,7 @@ static WaveLayout wave_layout(int64_t npixFrame, size_t ts, int aoN, bool needVo
   w.piters = take(iterFog && needVol ? (size_t)w.poolCap * kChunk * 4 : 0);
   w.segc = take(rays == 1 ? (size_t)((jobs + kHitSeg - 1) / kHitSeg) * kHitSegWarps * 4 : 0);
   w.hset = take(rays == 1 ? (size_t)npix * 8 * ts : 0);
+  w.colr = take(rays == 1 ? 5 * (size_t)npix * ts : 0);   // colour, normal (or its distances), fast AO
   w.total = off;
   return w;
 }
@@ -1175,6 +1176,10 @@ static int wave_occupancy(int formula, int block, int which) {
   if constexpr (sizeof(T) == 8) return occupancy_wave_f64(formula, block, which);
   else return occupancy_wave_f32(formula, block, which);
 }
+
+// Largest number of pixels x (1 + ray-AO directions) one wavefront group indexes with
+// 32-bit pixel and job numbers.
+constexpr double kMaxGroupJobs = 4.0e9;
 
 // Enqueue the wavefront stages (wave_core.cuh) of one group: primary rays, FP64 polish
 // (FP32 policy), shadow/AO rays, composition. No host round trips.
@@ -1310,6 +1315,13 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
   // as the device's launch sequence.
   const bool efx = rays > 1 || L.p.numberOfLights > 0 || L.p.volLightAny || L.p.iterFog || L.p.fakeLights;
   const bool secondaryJobs = scene.shadow != 0 || rayAO;
+  // the lean Mandelbulb's shadow stage runs the hits' colouring orbits and shading estimates too
+  // (secondary_lean), up to five more jobs per hit
+  const bool hitJobs = sizeof(T) == 4 && kf == 2 && L.fast && !efx && !L.p.slowShading && g.cfg.orbitRefill > 0 &&
+                       (double)g.npix * (6.0 + aoN) < kMaxGroupJobs;
+  wb.colour = hitJobs ? (T *)(base + w.colr) : nullptr;
+  wb.lean_normal = hitJobs ? wb.colour + g.npix : nullptr;
+  wb.lean_ao = hitJobs && scene.global_ilumination && scene.fastGlobalIllumination ? wb.colour + 4 * g.npix : nullptr;
   wb.hit_setup = (!efx && rays == 1 && secondaryJobs) ? (T *)(base + w.hset) : nullptr;
   cudaError_t e;
   if constexpr (sizeof(T) == 8) e = launch_wave_f64(L, s);
@@ -1482,9 +1494,6 @@ static mbgb_status check_opts(const mbgb_opts &o) {
   return MBGB_OK;
 }
 
-// Largest number of pixels x (1 + ray-AO directions) one wavefront group indexes with
-// 32-bit pixel and job numbers.
-constexpr double kMaxGroupJobs = 4.0e9;
 
 static void key_append(std::vector<char> &k, const void *p, size_t n) {
   k.insert(k.end(), (const char *)p, (const char *)p + n);

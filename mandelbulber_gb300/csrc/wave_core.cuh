@@ -104,22 +104,28 @@ struct LeanOrbit<8> {
   }
 };
 
+// The power-8 Mandelbulb's orbit also runs as the colouring orbit (start_colour): the same
+// iterations to |z| > 1e15 or `n` of them, with the smallest |z|^2 kept in minr2.
 template <>
 struct LeanOrbit<2> {
   static constexpr int kUnroll = 2;
-  float jx, jy, jz, cf, bail2;
+  float jx, jy, jz, cf, bailout2;
   int N;
   bool julia;
   float x, y, z, r2, r_dz, cx, cy, cz;
+  float bail2, minr2;   // of the current orbit
+  int n;
   int L;
   __device__ __forceinline__ explicit LeanOrbit(const FractalT<float> &f) {
     julia = f.juliaMode;
-    bail2 = f.bailout2;
+    bailout2 = f.bailout2;
     jx = f.julia[0]; jy = f.julia[1]; jz = f.julia[2];
     cf = f.constantFactor;
     N = f.N;
-    x = y = z = r2 = cx = cy = cz = 0.0f;
+    x = y = z = r2 = cx = cy = cz = minr2 = 0.0f;
     r_dz = 1.0f;
+    bail2 = bailout2;
+    n = N;
     L = 0;
   }
   __device__ __forceinline__ void start(const V3<float> p, const float) {
@@ -131,26 +137,45 @@ struct LeanOrbit<2> {
     x = p.x; y = p.y; z = p.z;
     r_dz = 1.0f;
     r2 = norm2_rn(x, y, z);
+    bail2 = bailout2;
+    n = N;
     L = 0;
   }
+  // at most `count` iterations
+  __device__ __forceinline__ void start(const V3<float> p, const float fparam, const int count) {
+    start(p, fparam);
+    n = count;
+  }
+  __device__ __forceinline__ void start_colour(const V3<float> p, const int n10) {
+    start(p, 0.0f);
+    bail2 = 1.0e30f;
+    n = n10;
+    minr2 = __int_as_float(0x7f800000);
+  }
+  // mandelbulb8_fast<1>'s value of an ended colouring orbit
+  __device__ __forceinline__ float colour_value() const { return (L < n ? sqrtf(minr2) : sqrtf(r2)) * 5000.0f; }
+  __device__ __forceinline__ float ended_dist() const {
+    const float r = sqrtf(r2);
+    return __fmul_rn(__fmul_rn(0.5f, r), __logf(r)) / r_dz;
+  }
   __device__ __forceinline__ bool advance(float &dist) {
-    if (L >= N) {
+    if (L >= n) {
       dist = 0.0f;
       return true;
     }
-    if (L <= N - kUnroll) {   // a whole block: the count is tested once, after it
+    if (L <= n - kUnroll) {   // a whole block: the count is tested once, after it
 #pragma unroll
       for (int u = 0; u < kUnroll; u++) {
         r2 = bulb8_iteration(x, y, z, r2, r_dz, cx, cy, cz);
+        minr2 = fminf(minr2, r2);
         if (r2 > bail2) {
           L += u;
-          const float r = sqrtf(r2);
-          dist = __fmul_rn(__fmul_rn(0.5f, r), __logf(r)) / r_dz;
+          dist = ended_dist();
           return true;
         }
       }
       L += kUnroll;
-      if (L == N) {
+      if (L == n) {
         dist = 0.0f;
         return true;
       }
@@ -159,12 +184,12 @@ struct LeanOrbit<2> {
 #pragma unroll 1
     for (;;) {
       r2 = bulb8_iteration(x, y, z, r2, r_dz, cx, cy, cz);
+      minr2 = fminf(minr2, r2);
       if (r2 > bail2) {
-        const float r = sqrtf(r2);
-        dist = __fmul_rn(__fmul_rn(0.5f, r), __logf(r)) / r_dz;
+        dist = ended_dist();
         return true;
       }
-      if (++L == N) {
+      if (++L == n) {
         dist = 0.0f;
         return true;
       }
@@ -280,13 +305,15 @@ __device__ __forceinline__ T wave_distance(const FractalT<T> &f, const V3<T> p, 
   return distance_est<T, FORMULA, FAST>(f, p, detail, N, minN, normalMode, L, maxIter, cnt, fparam);
 }
 
-// SurfaceColour (src/shaders.cpp:850-879) with the fast power-8 colouring orbit when it applies.
+// SurfaceColour (src/shaders.cpp:850-879) with the fast power-8 colouring orbit when it applies;
+// `value`: that orbit's value where the shadow stage has run it.
 template <typename T, int FORMULA, bool FAST>
 __device__ __forceinline__ V3<T> wave_colour(const ParamsT<T> &p, const V3<T> point, Counters &cnt,
-                                             const T fparam, const int objectType = kObjFractal) {
+                                             const T fparam, const int objectType = kObjFractal,
+                                             const T *value = nullptr) {
   if constexpr (FAST && FORMULA == 2 && sizeof(T) == 4) {
     int L;
-    const float c = mandelbulb8_fast<1>(p.f, point.x, point.y, point.z, p.f.N10, L, cnt);
+    const float c = value ? *value : mandelbulb8_fast<1>(p.f, point.x, point.y, point.z, p.f.N10, L, cnt);
     int nrCol = to_i32_x86((double)floorf(c));
     const unsigned mag = nrCol < 0 ? 0u - (unsigned)nrCol : (unsigned)nrCol;
     nrCol = (int)(mag % (248u * 256u));
@@ -2023,20 +2050,98 @@ __device__ __forceinline__ bool secondary_step(const ParamsT<T> &p, const WaveBu
   return done;
 }
 
+// The shading estimates of one hit of the lean Mandelbulb as a job of the orbit-granular shadow
+// stage (kind 4): CalculateNormals' four distances (calc_normal_fp), then FastAmbientOcclusion2's
+// quality^2 - 1 (wave_fast_ao), one orbit at a time, with the values and sums of those functions.
+// Without fast AO the four distances are four jobs (kind 5), since nothing follows them: a hit
+// whose orbits stay bounded would otherwise run 4 x 1250 iterations in a row, which bounded the
+// stage of a 640x480 frame (335 us of a 744 us frame; 700 us as four jobs).
+// s.j counts the orbits; s.end, s.maxSoft and s.stepMul hold the first three distances, s.r the
+// normal's step, s.dir the normal and s.sh the occlusion sum.
+__device__ __forceinline__ V3<float> shade_point(const ParamsT<float> &p, const SecondaryRay<float> &s) {
+  if (s.j == 0) return s.point;
+  if (s.j == 1) return V3<float>{s.point.x + s.r, s.point.y + 0.0f, s.point.z + 0.0f};
+  if (s.j == 2) return V3<float>{s.point.x + 0.0f, s.point.y + s.r, s.point.z + 0.0f};
+  if (s.j == 3) return V3<float>{s.point.x + 0.0f, s.point.y + 0.0f, s.point.z + s.r};
+  const int i = (int)s.j - 3;
+  const float scan = __fmul_rn(float(i * i), s.thr);
+  return V3<float>{fmaf(s.dir.x, scan, s.point.x), fmaf(s.dir.y, scan, s.point.y), fmaf(s.dir.z, scan, s.point.z)};
+}
+__device__ __forceinline__ void shade_begin(const ParamsT<float> &p, const WaveBufs<float> &wb,
+                                            const FrameCam<float> *__restrict__ cams, const int ncams,
+                                            const unsigned int k, SecondaryRay<float> &s) {
+  s.kind = 4;
+  s.j = 0;
+  s.gp = (int64_t)wb.hit_list[k];
+  const HitInfo<float> h = hit_info(p, cams[frame_of_pixel(cams, ncams, s.gp)], wb, s.gp);
+  s.point = h.point;
+  s.thr = h.thr;
+  s.detail = h.thr;
+  s.r = p.f.interiorMode ? h.thr * p.quality * 0.2f * p.smoothness : h.delta * p.smoothness;
+}
+// After orbit s.j's estimate (before CalculateDistance's clamps); true when the job has ended.
+__device__ __forceinline__ bool shade_step(const ParamsT<float> &p, const WaveBufs<float> &wb, SecondaryRay<float> &s,
+                                           const float odist, const int L) {
+  bool mi;
+  const bool normal = s.j < 4;
+  const float d = distance_post(p.f, odist, L, normal ? p.f.N5 : p.f.N, normal ? 0 : p.f.minN, s.detail, normal, 0.0f, mi);
+  if (s.j == 0) {
+    s.end = d;
+  } else if (s.j == 1) {
+    s.maxSoft = d;
+  } else if (s.j == 2) {
+    s.stepMul = d;
+  } else if (s.j == 3) {
+    V3<float> n{s.maxSoft - s.end, s.stepMul - s.end, d - s.end};
+    if (n.x == 0.0f && n.y == 0.0f && n.z == 0.0f) n.x = 1.0f;
+    else n = normalize3(n);
+    wb.lean_normal[s.gp] = n.x;
+    wb.lean_normal[wb.npix + s.gp] = n.y;
+    wb.lean_normal[2 * wb.npix + s.gp] = n.z;
+    s.dir = n;
+    s.sh = 0.0f;
+  } else {
+    const int i = (int)s.j - 3;
+    // the roundings of wave_fast_ao as it compiles: i^2 thr fused into the difference
+    const float w = i < 127 ? __uint_as_float((uint32_t)(127 - i) << 23) : i == 127 ? 5.877471754111438e-39f : 0.0f;
+    s.sh += __fdiv_rn(__fmul_rn(w, fmaf(float(i * i), s.thr, -__fmul_rn(p.fastAoTune, d))), s.thr);
+  }
+  s.j++;
+  if (s.j < 4) return false;
+  const unsigned int last = (p.ao && p.fastAO) ? 3u + (unsigned int)(p.aoQuality * p.aoQuality) : 4u;
+  if (s.j < last) return false;
+  if (p.ao && p.fastAO) {
+    float ao = __fsub_rn(1.0f, __fmul_rn(0.2f, s.sh));
+    if (ao < 0.0f) ao = 0.0f;
+    wb.lean_ao[s.gp] = ao;
+  }
+  return true;
+}
+
 // Lean FP32 orbits: lanes are refilled per orbit rather than per distance estimate. The
 // warp runs orbit iterations in batches of LeanOrbit::kUnroll until wb.orbit_refill of its
 // busy lanes have ended their orbits (or all have); then those lanes take their ray's next
 // step (or a new ray) and start the next orbit, while the others keep their orbit state.
 // Every distance is the one mandelbox_fast / mandelbulb8_fast returns at the same point.
+//
+// The Mandelbulb's stage also runs the hits' colouring orbits (kind 3) and shading estimates
+// (kind 4), first of all jobs (wb.colour). Estimate by estimate in the composition, whose warps
+// wait for their longest orbit (4 to 1250 iterations; 2500 for the colour), they ran at 8.2
+// active lanes of 32. Eight flight frames 14.2 -> 10.7 ms
+// (13.8 - 15.9 at the start by views), identical layers. Their counts go to the composition's counters.
 template <int FORMULA>
 __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const FrameIO &io, const WaveBufs<float> &wb,
                                                const FrameCam<float> *__restrict__ cams, const int ncams) {
   const unsigned int nh = *(volatile unsigned int *)&wb.ctl[1];
   const SecondaryJobs jn = secondary_jobs(p, wb, nh);
-  const unsigned int njobs = jn.nShadow + jn.nAO + jn.nAux;
+  // colours, then shadings (with fast AO) or normal distances
+  const unsigned int nHitJobs = (FORMULA == 2 && wb.colour) ? (wb.lean_ao ? 2u : 5u) * nh : 0u;
+  const unsigned int njobs = nHitJobs + jn.nShadow + jn.nAO + jn.nAux;
   const unsigned int threshold = (unsigned int)wb.orbit_refill;
   const int minN = p.f.minN;
   Counters cnt{0, 0, 0, 0};
+  unsigned long long hitOrbit = 0;   // of the hit jobs
+  unsigned int hitCalls = 0;
   LeanOrbit<FORMULA> orb(p.f);
   SecondaryRay<float> s{};
   bool active = false, exhausted = job_share(wb, njobs).idle, orbiting = false;
@@ -2044,15 +2149,36 @@ __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const Fr
   for (;;) {
     // lanes whose orbit ended: the distance estimate's clamps, then the ray's step
     if (active && !orbiting) {
-      cnt.orbit += (unsigned long long)(orb.L + 1);
-      cnt.calls += 1;
-      bool mi;
-      const float d = distance_post(p.f, odist, orb.L, orb.N, minN, s.detail, false, 0.0f, mi);
-      if (secondary_step(p, wb, s, d, mi)) {
-        active = false;
+      if (FORMULA == 2 && s.kind >= 3) {
+        hitOrbit += (unsigned long long)(orb.L + 1);
+        hitCalls++;
+        if constexpr (FORMULA == 2) {
+          if (s.kind == 3) {
+            wb.colour[s.gp] = orb.colour_value();
+            active = false;
+          } else if (s.kind == 5) {
+            bool mi;
+            wb.lean_normal[(int64_t)s.j * wb.npix + s.gp] =
+                distance_post(p.f, odist, orb.L, p.f.N5, 0, s.detail, true, 0.0f, mi);
+            active = false;
+          } else if (shade_step(p, wb, s, odist, orb.L)) {
+            active = false;
+          } else {
+            orb.start(shade_point(p, s), 0.0f, s.j < 4 ? p.f.N5 : p.f.N);
+            orbiting = true;
+          }
+        }
       } else {
-        orb.start(ray_at(s.point, s.dir, s.r), s.fpar);
-        orbiting = true;
+        cnt.orbit += (unsigned long long)(orb.L + 1);
+        cnt.calls += 1;
+        bool mi;
+        const float d = distance_post(p.f, odist, orb.L, orb.N, minN, s.detail, false, 0.0f, mi);
+        if (secondary_step(p, wb, s, d, mi)) {
+          active = false;
+        } else {
+          orb.start(ray_at(s.point, s.dir, s.r), s.fpar);
+          orbiting = true;
+        }
       }
     }
     // idle lanes take new rays until every lane is busy or the jobs are spent
@@ -2066,7 +2192,25 @@ __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const Fr
       if (need) {
         if (stop || job >= njobs) {
           exhausted = true;
-        } else if (secondary_begin(p, wb, cams, ncams, nh, jn, job, s)) {
+        } else if (job < nHitJobs) {
+          if constexpr (FORMULA == 2) {
+            if (job < nh) {
+              s.kind = 3;
+              s.gp = (int64_t)wb.hit_list[job];
+              orb.start_colour(V3<float>{wb.point[s.gp], wb.point[wb.npix + s.gp], wb.point[2 * wb.npix + s.gp]}, p.f.N10);
+            } else {
+              const unsigned int q = job / nh;   // 1, or 1 to 4
+              shade_begin(p, wb, cams, ncams, job - q * nh, s);
+              if (!wb.lean_ao) {
+                s.kind = 5;
+                s.j = q - 1u;
+              }
+              orb.start(shade_point(p, s), 0.0f, p.f.N5);
+            }
+            active = true;
+            orbiting = true;
+          }
+        } else if (secondary_begin(p, wb, cams, ncams, nh, jn, job - nHitJobs, s)) {
           active = true;
           orb.start(ray_at(s.point, s.dir, s.r), s.fpar);
           orbiting = true;
@@ -2085,10 +2229,16 @@ __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const Fr
   for (int off = 16; off > 0; off >>= 1) {
     cnt.orbit += __shfl_down_sync(0xffffffffu, cnt.orbit, off);
     cnt.calls += __shfl_down_sync(0xffffffffu, cnt.calls, off);
+    hitOrbit += __shfl_down_sync(0xffffffffu, hitOrbit, off);
+    hitCalls += __shfl_down_sync(0xffffffffu, hitCalls, off);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicAdd(&io.counters[0], cnt.orbit);
     atomicAdd(&io.counters[1], cnt.calls);
+    if (nHitJobs) {   // the composition stage's counters
+      atomicAdd(&io.counters[4], hitOrbit);
+      atomicAdd(&io.counters[5], (unsigned long long)hitCalls);
+    }
   }
 }
 
@@ -2566,6 +2716,13 @@ __device__ __forceinline__ void shade_hit(const ParamsT<T> &p, const FrameCam<T>
     nrm = *slowSum;
     if (nrm.x == T(0) && nrm.y == T(0) && nrm.z == T(0)) nrm.x = T(1);
     else nrm = normalize3(nrm);
+  } else if (!EFX && wb.lean_normal && !wb.lean_ao) {   // from the shadow stage's four distances
+    const T s1 = wb.lean_normal[ri];
+    nrm = {wb.lean_normal[wb.npix + ri] - s1, wb.lean_normal[2 * wb.npix + ri] - s1, wb.lean_normal[3 * wb.npix + ri] - s1};
+    if (nrm.x == T(0) && nrm.y == T(0) && nrm.z == T(0)) nrm.x = T(1);
+    else nrm = normalize3(nrm);
+  } else if (!EFX && wb.lean_normal) {   // computed by the shadow stage (secondary_lean)
+    nrm = {wb.lean_normal[ri], wb.lean_normal[wb.npix + ri], wb.lean_normal[2 * wb.npix + ri]};
   } else if (EFX && wb.normal) {   // computed by the normal stage (auxiliary lights)
     nrm = {wb.normal[ri], wb.normal[wb.npix + ri], wb.normal[2 * wb.npix + ri]};
   } else {
@@ -2582,7 +2739,8 @@ __device__ __forceinline__ void shade_hit(const ParamsT<T> &p, const FrameCam<T>
   shade2 = m_pow(shade2, T(30)) * T(1);
   if (shade2 > T(15)) shade2 = T(15);
   const T specT = shade2 * p.specular;
-  const V3<T> colour = wave_colour<T, FORMULA, FAST>(p, h.point, cnt, c.fparam, objectType);
+  const V3<T> colour = wave_colour<T, FORMULA, FAST>(p, h.point, cnt, c.fparam, objectType,
+                                                     !EFX && wb.colour ? wb.colour + ri : nullptr);
   colourOut = colour;
   V3<T> ambient{T(0), T(0), T(0)};
   if (p.ao) {
@@ -2591,7 +2749,8 @@ __device__ __forceinline__ void shade_hit(const ParamsT<T> &p, const FrameCam<T>
       const T factor = p.penetrating ? h.delta / c.resolution : p.viewDistanceMax;
       const T shadowStart = p.f.interiorMode ? h.thr * p.DE_factor : h.thr;
       const T detail = (p.shadow && shadowStart < factor) ? (T)(float)h.thr : h.thr;
-      const T a = wave_fast_ao<T, FORMULA, FAST>(p, h.point, nrm, h.thr, detail, cnt, c.fparam);
+      const T a = !EFX && wb.lean_ao ? wb.lean_ao[ri]
+                                     : wave_fast_ao<T, FORMULA, FAST>(p, h.point, nrm, h.thr, detail, cnt, c.fparam);
       ambient = {a, a, a};
     } else {
       T acc = T(0);
@@ -2622,6 +2781,24 @@ __device__ __forceinline__ void shade_hit(const ParamsT<T> &p, const FrameCam<T>
     // no auxiliary or fake lights: their specular terms are the reference's zeros
     for (int k = 0; k < 3; k++) spec[k] = T(0) + p.mainLight[k] * specT * shadow;
   }
+}
+
+// to_u16_x86(v * 65535.0) and to_u8_x86(v) of the layers' values. In FP32 without the FP64 pipe,
+// whose conversions and products took 20 SM cycles each (the Mandelbulb's composition was bound by
+// them): the 24-bit product by 65535 is exact in 64-bit integers, and a float's conversion to
+// int32 truncates as the double's does.
+__device__ __forceinline__ uint16_t u16_of(const double v) { return to_u16_x86(v * 65535.0); }
+__device__ __forceinline__ uint16_t u16_of(const float v) {
+  // |v| x 65535 at 2^31 and above (and NaN) is cvttsd2si's INT_MIN, whose low 16 bits are 0
+  const uint32_t b = __float_as_uint(v), e = (b >> 23) & 0xffu;
+  if (e < 110u || !(fabsf(v) <= 32768.5f)) return 0;
+  const uint64_t prod = (uint64_t)((b & 0x7fffffu) | 0x800000u) * 65535u;
+  const uint32_t q = e <= 150u ? (uint32_t)(prod >> (150u - e)) : (uint32_t)(prod << (e - 150u));
+  return (uint16_t)(v < 0.0f ? 0u - q : q);
+}
+__device__ __forceinline__ uint8_t u8_of(const double v) { return to_u8_x86(v); }
+__device__ __forceinline__ uint8_t u8_of(const float v) {
+  return (uint8_t)(v >= -2147483648.0f && v < 2147483648.0f ? __float2int_rz(v) : (int)0x80000000);
 }
 
 // ---------------------------------------------------------------------------
@@ -2745,8 +2922,8 @@ __global__ void __launch_bounds__(128, (FAST && sizeof(T) == 4) ? 10 : 1) compos
     out2 = result[2];
     const bool hit = (wb.flags[gp] & 1) != 0;
     const double depth = hit ? (double)wb.scan[gp] : 1e20;
-    if (c.opacity) c.opacity[pix] = to_u16_x86((double)opacity * 65535.0);
-    if (c.alpha) c.alpha[pix] = to_u16_x86((double)alpha * 65535.0);
+    if (c.opacity) c.opacity[pix] = u16_of(opacity);
+    if (c.alpha) c.alpha[pix] = u16_of(alpha);
     if (c.zbuffer) c.zbuffer[pix] = (float)depth;
     // debug layer: 0 miss, 1 hit, 3 hit whose exact_hit refinement missed the level set
     if (c.hit) c.hit[pix] = hit ? ((wb.flags[gp] & 8) ? 3 : 1) : 0;
@@ -2760,8 +2937,7 @@ __global__ void __launch_bounds__(128, (FAST && sizeof(T) == 4) ? 10 : 1) compos
     const bool aligned = (!c.image_float || ((uintptr_t)(c.image_float + 3 * pix0) & 15u) == 0) &&
                          (!c.colour || ((uintptr_t)(c.colour + 3 * pix0) & 15u) == 0);
     const bool vec = __all_sync(0xffffffffu, valid && c.pixBase == base0 && aligned);
-    const uint8_t col[3] = {to_u8_x86((double)(objColour.x * T(255))), to_u8_x86((double)(objColour.y * T(255))),
-                            to_u8_x86((double)(objColour.z * T(255)))};
+    const uint8_t col[3] = {u8_of(objColour.x * T(255)), u8_of(objColour.y * T(255)), u8_of(objColour.z * T(255))};
     if (vec) {
       // 32 pixels x 12 bytes = 24 float4 stores, 32 x 3 bytes = 6 uint4 stores
       float *si = stageImg[warp];

@@ -24,6 +24,11 @@ struct WaveBufs {
   T *vol;                // [6][npix] overflow pass only: A, B.r, B.g, B.b, alpha, opacity
   T *shadow;             // [npix]
   T *ao;                 // [aoCount][npix] per-direction shadowTemp
+  // what the shadow stage of the lean Mandelbulb with orbit-granular refill computes of each hit
+  // (null: the composition does)
+  T *colour;             // [npix] the colouring orbit's value
+  T *lean_normal;        // [3][npix] the normal, or without fast AO [4][npix] its four distances
+  T *lean_ao;            // [npix] fast AO (null without)
   T *normal;             // [3][npix] hit normals (auxiliary lights: null without them)
   T *auxsh;              // [numberOfLights][npix] AuxShadow of each auxiliary light at each hit
                          // (null without aux lights or shadows)

@@ -2,7 +2,7 @@
 // results bit for bit at a third of the FP64 instructions of compute<double, 8, 0>.
 //
 // What bounds it: GB300's FP64 pipe, 20 SM cycles per warp instruction (exact64.cuh). The
-// generic iteration (tglad_step) issues 61 of them; here the usual iteration issues 11, beside
+// generic iteration (tglad_step) issues 61 of them; here the usual iteration issues 8, beside
 // integer work of about as many cycles:
 //   * The orbit needs r = sqrt(q), q = |z|^2, only inside the sphere fold's shell. The tests
 //     r * r < mR2, r * r < fR2 and r > 1024 are monotone in q (square root and product round
@@ -16,8 +16,9 @@
 //     two roundings.
 //   * The fold against a power of two, the squares before the sphere fold and the shell's
 //     products are integer too: moving them off the pipe took 2 M orbits of 15 iterations from
-//     1.53 to 1.07 ms (fold 1.53 -> 1.33, products -> 1.17, squares -> 1.07); moving the
-//     bailout's squares as well made it 1.11, so they stay.
+//     1.53 to 1.07 ms (fold 1.53 -> 1.33, products -> 1.17, squares -> 1.07). The bailout's
+//     squares too: 25.3 -> 23.2 ms for a frame, whose stages have fewer active lanes and free issue
+//     slots, but 1.07 -> 1.11 ms for that loop of full warps, which keeps them (FULL).
 // Measured: 2,000,003 distances (N 15) 3.92 ms generic, 1.44 ms with the pipe for fold and
 // products, 0.96 ms as it stands; a 481x271 Mandelbox frame 92.9 -> 28.0 ms.
 // Not kept: leaving out the bailout test of the first five iterations, which a start point near
@@ -50,6 +51,8 @@ __device__ __forceinline__ double box_dist_strict(const double q, const double d
   return div_exact(sqrt_exact(q), dr);
 }
 
+// FULL: the caller's warps are full (a point cloud): the bailout's squares stay on the pipe.
+template <bool FULL>
 __device__ __forceinline__ double box_orbit_strict(const FractalT<double> &f, double x, double y, double z,
                                                    const double cx, const double cy, const double cz, const int N,
                                                    int &Lout, const double scale) {
@@ -102,7 +105,8 @@ __device__ __forceinline__ double box_orbit_strict(const FractalT<double> &f, do
       z = __dadd_rn(__dmul_rn(z, scale), cz);
       dr = __dadd_rn(__dmul_rn(dr, fabs(scale)), 1.0);
     }
-    const double q2 = norm2_strict(x, y, z);
+    const double q2 = FULL ? norm2_strict(x, y, z)
+                           : __dadd_rn(__dadd_rn(square_int(x), square_int(y)), square_int(z));
     if (f64_bits(q2) > qBail) {
       Lout = L;
       return box_dist_strict(q2, dr);

@@ -268,13 +268,14 @@ __device__ __forceinline__ float mandelbox_fast(const FractalT<float> &f, const 
 }
 
 // The FP64 Mandelbox orbit (formula 8, normal mode) through box_orbit_strict.
+template <bool FULL>
 __device__ __forceinline__ double mandelbox_strict(const FractalT<double> &f, const V3<double> p, const int N,
                                                    int &Lout, Counters &cnt, const double scale) {
   const V3<double> c = f.juliaMode ? V3<double>{f.julia[0], f.julia[1], f.julia[2]}
                                    : V3<double>{__dmul_rn(p.x, f.constantFactor), __dmul_rn(p.y, f.constantFactor),
                                                 __dmul_rn(p.z, f.constantFactor)};
   int L;
-  const double dist = box_orbit_strict(f, p.x, p.y, p.z, c.x, c.y, c.z, N, L, scale);
+  const double dist = box_orbit_strict<FULL>(f, p.x, p.y, p.z, c.x, c.y, c.z, N, L, scale);
   cnt.orbit += (unsigned long long)(L + 1);
   cnt.calls += 1;
   Lout = L;
@@ -417,7 +418,8 @@ __device__ __forceinline__ T distance_post(const FractalT<T> &f, T distance, con
 
 // CalculateDistance, analytic branch (src/fractal.cpp:1245-1300, 1436-1445).
 // `L` (itersOut) is left untouched when the limits box returns early, as in the reference.
-template <typename T, int FORMULA>
+// FULL: box_orbit_strict's form for full warps.
+template <typename T, int FORMULA, bool FULL = false>
 __device__ __forceinline__ T calc_distance(const FractalT<T> &f, const V3<T> point, const T detailSize, const int N,
                                            const int minN, const bool normalMode, int &L, bool &maxIter,
                                            Counters &cnt, const T fparam) {
@@ -443,7 +445,7 @@ __device__ __forceinline__ T calc_distance(const FractalT<T> &f, const V3<T> poi
     }
   } else if constexpr (kStrictF64 && sizeof(T) == 8 && FORMULA == 8) {
     distance = f.boxStrict && box_strict_point(point.x, point.y, point.z)
-                   ? mandelbox_strict(f, point, N, Li, cnt, fparam)
+                   ? mandelbox_strict<FULL>(f, point, N, Li, cnt, fparam)
                    : compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
   } else {
     distance = compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
@@ -1648,7 +1650,7 @@ __global__ void distance_kernel(const __grid_constant__ FractalT<T> f, const dou
     const V3<T> pt{(T)points[3 * i], (T)points[3 * i + 1], (T)points[3 * i + 2]};
     int L = 0;
     bool mi = false;
-    const T d = calc_distance<T, FORMULA>(f, pt, (T)detail[i], f.N, f.minN, false, L, mi, cnt, fparam_of(f));
+    const T d = calc_distance<T, FORMULA, true>(f, pt, (T)detail[i], f.N, f.minN, false, L, mi, cnt, fparam_of(f));
     dist[i] = (double)d;
     iters[i] = L;
     max_iter[i] = mi ? 1 : 0;

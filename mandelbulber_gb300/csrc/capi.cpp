@@ -332,6 +332,17 @@ static void fill_box_strict(const mbgb_scene &s, FractalT<T> &f) {
   if (fv > 1e-60 && frexp(fv, &e) == 0.5 && 2.0 * s.mboxFoldingLimit >= fv) f.boxFoldFar = (T)ldexp(fv, 50);
 }
 
+// FractalT::leanFreeR2 for a scene's own scale. The box fold lengthens no component and the
+// sphere fold leaves max(r, fR^2 / mR) at most, so r' <= |s| max(r, fR^2 / mR) + |c|: after five
+// iterations |s|^5 max(|p|, fR^2 / mR) + |c| (1 + |s| + ... + |s|^4), |c| = |constant factor| |p|,
+// held to 1000 of the bailout's 1024 (FP32 rounding is 1e-6 of it).
+static double box_free_r2(const mbgb_scene &s) {
+  const double a = std::max(fabs(s.mboxScale), 1.0), a2 = a * a, a4 = a2 * a2;
+  const double p = 1000.0 / (a4 * a + fabs(s.constantFactor) * (1.0 + a + a2 + a2 * a + a4));
+  const double shell = s.mboxFoldingSphericalFixed * s.mboxFoldingSphericalFixed / fabs(s.mboxFoldingSphericalMin);
+  return fast_mandelbox(s) && s.mboxFoldingLimit >= 0.0 && p >= shell ? p * p : -1.0;   // (false for NaN)
+}
+
 template <typename T>
 static void fill_fractal(const mbgb_scene &s, FractalT<T> &f) {
   memset(&f, 0, sizeof(f));
@@ -375,6 +386,7 @@ static void fill_fractal(const mbgb_scene &s, FractalT<T> &f) {
     f.leanSa = km1 > T(0) ? fR2 / km1 : T(0);
     f.leanSb = km1 > T(0) ? T(1) / km1 : T(0);
   }
+  f.leanFreeR2 = (T)box_free_r2(s);
   if (sizeof(T) == 8) fill_box_strict(s, f);
   if (sizeof(T) == 8 && !s.analitycDE && s.formula >= 3 && s.formula <= 6 && !s.ifsFoldingMode &&
       !s.tgladFoldingMode && !s.sphericalFoldingMode) {
@@ -934,6 +946,7 @@ template <typename T>
 static void clear_fparam(FractalT<T> &f) {
   if (scale_formula_host(f.formula)) f.mbScale = T(0);
   else f.power = T(0);
+  f.leanFreeR2 = T(0);   // follows the scale: a launch takes its frames' smallest
 }
 
 // Whether frames a and b can share one launch sequence in precision T: every
@@ -1306,6 +1319,7 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
   L.fast = (fast_mandelbox(scene) || fast_mandelbulb(scene)) && !scene.limits_enabled;
   fill_fractal<double>(scene, L.fd);
   fill_params<T>(scene, L.p, o, (const T *)(prec == 0 ? c->ao64.ptr : c->ao32.ptr), c->ao_count);
+  for (int i : g.frames) L.p.f.leanFreeR2 = std::min(L.p.f.leanFreeR2, (T)box_free_r2(scenes[i]));
   if (lightOff >= 0)
     L.p.lights = (const LightT<T> *)(prec == 0 ? c->lights64.ptr : c->lights32.ptr) + lightOff;
   else if (auxN > 0)

@@ -63,6 +63,8 @@ struct FractalT {
   // lean Mandelbox sphere fold, derived on the host in T's arithmetic: k1 - 1 = fR^2/mR^2 - 1,
   // fR^2/(k1 - 1) and 1/(k1 - 1) (0 when k1 <= 1)
   T leanKm1, leanSa, leanSb;
+  T leanFreeR2;     // |p|^2 up to which a lean Mandelbox orbit cannot pass the bailout in its first
+                    // kBoxBlock iterations (-1: none)
   // FP64 Mandelbox without rotations, offset or pre-folds (box_orbit_strict, lean_orbit64.cuh):
   // whether it applies, and its bounds on |z|^2: r * r < mR2, r * r < fR2 and r > 1024 hold
   // exactly where |z|^2 < boxQIn, < boxQMid and > boxQBail; fR2 / mR2 and whether that is a

@@ -260,7 +260,7 @@ __device__ __forceinline__ float mandelbox_fast(const FractalT<float> &f, const 
   const float cx = __fmul_rn(px, f.constantFactor), cy = __fmul_rn(py, f.constantFactor),
               cz = __fmul_rn(pz, f.constantFactor);
   int L;
-  const float dist = box_orbit(k, s, skm1, px, py, pz, cx, cy, cz, N, L);
+  const float dist = box_orbit(k, s, skm1, px, py, pz, cx, cy, cz, N, L, f.leanFreeR2);
   cnt.orbit += (unsigned long long)(L + 1);
   cnt.calls += 1;
   Lout = L;

@@ -13,7 +13,7 @@ namespace dev {
 template <typename T, int K>
 struct Dual {
   T v;
-  T d[K];
+  T d[K > 0 ? K : 1];   // (K = 0: the value alone, through the same operations)
 };
 
 template <typename T, int K>
@@ -213,7 +213,7 @@ __device__ __forceinline__ Dual<T, K> de_dual_seeded(const FractalT<T> &f, DV3<T
     D r_dz = dconst<T, K>(T(1));
     // FP32: the running derivative's tangents grow like r_dz^2 and leave FP32's range near
     // the surface, so they are carried relative to r_dz (q = d r_dz / r_dz), which stays small
-    T rdz = T(1), q[K];
+    T rdz = T(1), q[K > 0 ? K : 1];
 #pragma unroll
     for (int k = 0; k < K; k++) q[k] = T(0);
     for (L = 0; L < N; L++) {
@@ -309,15 +309,33 @@ __device__ __forceinline__ Dual<T, 1> de_along(const FractalT<T> &f, const V3<T>
   return de_dual_seeded<T, FORMULA, 1>(f, z, dconst<T, 1>(fparam), N, Lout);
 }
 
+// Whether the orbit of P escapes within N iterations: de_along's value without its tangents.
+template <typename T, int FORMULA>
+__device__ __forceinline__ bool escapes(const FractalT<T> &f, const V3<T> P, const int N, const T fparam) {
+  DV3<T, 0> z;
+  z.x.v = P.x;
+  z.y.v = P.y;
+  z.z.v = P.z;
+  Dual<T, 0> fp;
+  fp.v = fparam;
+  int L;
+  de_dual_seeded<T, FORMULA, 0>(f, z, fp, N, L);
+  return L < N;
+}
+
 // Newton refinement of a hit to the level set DE(o + t d) = thr(t) in FP64 (after the
 // reference's binary refinement has put it inside the window (0.99 thr, thr)). Returns
 // false (and leaves t) when the level set is not reached: a grazing ray (F_t >= 0), a
 // flat estimate (orbit not escaping, minN clamp), or no convergence in 16 steps.
+// `bounded`: the FP32 refinement met an orbit that did not escape. Such a hit usually fails here
+// for the same reason after N iterations of the pipe-bound libm orbit, and its chain bounds the
+// stage, so the orbit is first run without tangents. Eight 256x256 frames 6.24 -> 5.91 ms.
 template <int FORMULA>
 __device__ __forceinline__ bool level_set_hit(const FractalT<double> &f, const V3<double> o, const V3<double> d,
                                               const double k, const double thrConst, double &t, int &iters,
-                                              const double fparam) {
+                                              const double fparam, const bool bounded) {
   double tt = t;
+  if (bounded && !escapes<double, FORMULA>(f, o + d * tt, f.N, fparam)) return false;
   for (int it = 0; it < 16; it++) {
     int L;
     const Dual<double, 1> de = de_along<double, FORMULA>(f, o + d * tt, d, f.N, L, fparam);
@@ -347,13 +365,14 @@ __device__ __forceinline__ bool level_set_hit(const FractalT<double> &f, const V
 template <int FORMULA>
 __device__ __forceinline__ bool level_set_hit_f32(const FractalT<float> &f, const V3<float> o, const V3<float> d,
                                                   const float k, const float thrConst, float &t, int &iters,
-                                                  const float fparam) {
+                                                  const float fparam, bool &bounded) {
   float tt = t;
   const float lenD = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
   for (int it = 0; it < 16; it++) {
     int L;
     const Dual<float, 1> de = de_along<float, FORMULA>(f, o + d * tt, d, f.N, L, fparam);
     const float thr = k > 0.0f ? tt * k : thrConst;
+    if (L == f.N) bounded = it == 0;
     if (L == f.N || L < f.minN || !isfinite(de.v) || !isfinite(de.d[0])) return false;
     const float F = de.v - thr;
     if (fabsf(F) <= 2e-5f * thr) {

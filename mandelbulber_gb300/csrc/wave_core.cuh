@@ -2905,8 +2905,11 @@ __device__ __forceinline__ uint8_t u8_of(const float v) {
 // Stage 4: per-pixel composition and the cImage writes (src/Render3D.cpp:501-589),
 // over every pixel of the batch.
 // ---------------------------------------------------------------------------
+// The FP32 effects variant is bounded by latency (17 % issue at 5 warps per SM with its 215
+// registers): held to 5 blocks per SM, 480x270 Menger sponge with lights and reflections 8.63 ->
+// 7.76 ms (3: 8.13, 4: 8.09, 6: 7.77, 8: 8.10).
 template <typename T, int FORMULA, bool FAST, bool EFX = false>
-__global__ void __launch_bounds__(128, (FAST && sizeof(T) == 4) ? 10 : 1) compose_kernel(const __grid_constant__ ParamsT<T> p, const FrameIO io, const WaveBufs<T> wb,
+__global__ void __launch_bounds__(128, (FAST && sizeof(T) == 4) ? 10 : (EFX && sizeof(T) == 4) ? 5 : 1) compose_kernel(const __grid_constant__ ParamsT<T> p, const FrameIO io, const WaveBufs<T> wb,
                                                       const FrameCam<T> *__restrict__ cams, const int ncams) {
   Counters cnt{0, 0, 0, 0};
   const int64_t total = wb.npix_frame;

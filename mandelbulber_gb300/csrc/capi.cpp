@@ -747,6 +747,8 @@ struct CallPlan {
   bool grad = false;             // the gradient stage runs after composition
 };
 
+constexpr size_t kControlBytes = 256;
+
 struct mbgb_context {
   int device = 0;
   int sms = 0;
@@ -754,8 +756,12 @@ struct mbgb_context {
   DeviceBuf step[2][5];          // per-pixel engine: [precision][step, dist, thr, scan, iters], kStepCap records per slot
   DeviceBuf ovstep[2][5];        // overflow passes: kStepSlots records per slot and ray
   DeviceBuf ovlist;              // overflow pixel list (per-pixel engine)
-  DeviceBuf control;             // error flag, start time, stage counters
-  DeviceBuf fctl;                // per group: wavefront stage counters / per-pixel tile counter (64 B each)
+  // error flag, start time and stage counters (kControlBytes), then per group the wavefront's stage
+  // counters / the per-pixel engine's tile counter (64 B each): one buffer, zeroed by one memset
+  // before a call's launches and read back by one copy after them
+  DeviceBuf control;
+  char *status = nullptr;        // pinned host copy of `control`
+  size_t status_bytes = 0;
   DeviceBuf cams;                // frame tables of the wavefront groups
   DeviceBuf ao64, ao32;
   int ao_quality = -1;
@@ -862,7 +868,7 @@ extern "C" void mbgb_context_destroy(mbgb_context *c) {
   c->gradacc.release();
   c->post.release();
   c->control.release();
-  c->fctl.release();
+  if (c->status) cudaFreeHost(c->status);
   c->cams.release();
   if (c->graph) cudaGraphExecDestroy(c->graph);
   for (auto ev : c->gev)
@@ -1271,7 +1277,6 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
   // shadow/AO rays two per thread (secondary_pair_kernel): the lean FP32 Mandelbox with
   // per-estimate refill, which the pair kernel's packed orbit serves
   wb.pair_rays = (sizeof(T) == 4 && fast_mandelbox(scene) && g.cfg.pairRays && g.cfg.orbitRefill <= 0) ? 1 : 0;
-  MBGB_CUDA(cudaMemsetAsync(ctl, 0, 64, s));
 
   const int block = g.cfg.block;
   const int kf = distance_kernel_formula(scene);
@@ -1410,7 +1415,6 @@ static mbgb_status enqueue_per_pixel(mbgb_context *c, const mbgb_scene &scene, c
     io.step_iters = points ? (int *)c->step[prec][4].ptr : nullptr;
     io.overflow_list = (unsigned int *)c->ovlist.ptr;
   }
-  MBGB_CUDA(cudaMemsetAsync(fctl, 0, 64, s));
   FrameIO ov = io;
   ov.overflow_pass = 1;
   ov.step_cap = kStepSlots;
@@ -1843,8 +1847,15 @@ static mbgb_status render_frames(mbgb_context *c, const mbgb_scene *scenes, int 
         MBGB_CUDA(c->ensure(c->step[p][k], (size_t)kStepCap * (size_t)maxSlots[p] * bytes_of(k)));
   }
   if (maxPixPerPixel) MBGB_CUDA(c->ensure(c->ovlist, (size_t)maxPixPerPixel * sizeof(unsigned int)));
-  MBGB_CUDA(c->ensure(c->control, 256));
-  MBGB_CUDA(c->ensure(c->fctl, 64 * plan.groups.size()));
+  const size_t controlBytes = kControlBytes + 64 * plan.groups.size();
+  MBGB_CUDA(c->ensure(c->control, controlBytes));
+  if (c->status_bytes < controlBytes) {
+    if (c->status) cudaFreeHost(c->status);
+    c->status = nullptr;
+    c->status_bytes = 0;
+    MBGB_CUDA(cudaMallocHost((void **)&c->status, controlBytes));
+    c->status_bytes = controlBytes;
+  }
   if (grad) MBGB_CUDA(c->ensure(c->gradacc, sizeof(double) * kGradParams * (size_t)n));
   std::vector<char> camsHost(camsBytes);
   for (auto &g : plan.groups) {
@@ -1939,11 +1950,11 @@ static mbgb_status render_frames(mbgb_context *c, const mbgb_scene *scenes, int 
   io.counters = (unsigned long long *)(ctl + 64);
   io.budget_ns = o.deadline_ms > 0 ? (unsigned long long)o.deadline_ms * 1000000ull : 0ull;
   auto enqueue = [&]() -> mbgb_status {
-    MBGB_CUDA(cudaMemsetAsync(ctl, 0, 256, s));
+    MBGB_CUDA(cudaMemsetAsync(ctl, 0, controlBytes, s));
     if (grad) MBGB_CUDA(cudaMemsetAsync(c->gradacc.ptr, 0, sizeof(double) * kGradParams * (size_t)n, s));
     for (size_t gi = 0; gi < plan.groups.size(); gi++) {
       const Group &g = plan.groups[gi];
-      char *gctl = (char *)c->fctl.ptr + 64 * gi;
+      char *gctl = ctl + kControlBytes + 64 * gi;
       cudaEvent_t *ev = plan.profile ? &c->gev[kStageEvents * gi] : nullptr;
       mbgb_status r;
       if (!g.wave) {
@@ -2002,16 +2013,17 @@ static mbgb_status render_frames(mbgb_context *c, const mbgb_scene *scenes, int 
 // Wait for the call's stream and fill the context's counters (the reference's globals,
 // src/Render3D.cpp:51-57) from the device.
 static mbgb_status read_back(mbgb_context *c, const CallPlan &plan, int replayed) {
+  // one copy behind the launches and one wait (three synchronous copies after a wait took 30 us of
+  // a 160x120 frame's 226)
+  const size_t bytes = kControlBytes + 64 * plan.groups.size();
+  MBGB_CUDA(cudaMemcpyAsync(c->status, c->control.ptr, bytes, cudaMemcpyDeviceToHost, c->stream));
   MBGB_CUDA(cudaStreamSynchronize(c->stream));
-  MBGB_CUDA(cudaEventSynchronize(c->ev1));
-  char *ctl = (char *)c->control.ptr;
   unsigned long long cnt[4 * kStages];
   int flag = 0;
-  MBGB_CUDA(cudaMemcpy(cnt, ctl + 64, sizeof(cnt), cudaMemcpyDeviceToHost));
-  MBGB_CUDA(cudaMemcpy(&flag, ctl + 16, sizeof(flag), cudaMemcpyDeviceToHost));
+  memcpy(cnt, c->status + 64, sizeof(cnt));
+  memcpy(&flag, c->status + 16, sizeof(flag));
   std::vector<uint32_t> gctl(16 * plan.groups.size());
-  if (!gctl.empty())
-    MBGB_CUDA(cudaMemcpy(gctl.data(), c->fctl.ptr, 64 * plan.groups.size(), cudaMemcpyDeviceToHost));
+  if (!gctl.empty()) memcpy(gctl.data(), c->status + kControlBytes, 64 * plan.groups.size());
   mbgb_stats &S = c->stats;
   S = mbgb_stats{};
   for (int k = 0; k < kStages; k++) {

@@ -106,9 +106,11 @@ struct LeanOrbit<8> {
 
 // The power-8 Mandelbulb's orbit also runs as the colouring orbit (start_colour): the same
 // iterations to |z| > 1e15 or `n` of them, with the smallest |z|^2 kept in minr2.
+// Batches of 4 iterations against 2: 640x480 Mandelbulb 598 -> 551 us, eight flight frames 12.7 ->
+// 12.0 ms (3: 571 us, 12.3 ms), with 8 ended orbits before the warp steps on (4 to 24: within 3 %).
 template <>
 struct LeanOrbit<2> {
-  static constexpr int kUnroll = 2;
+  static constexpr int kUnroll = 4;
   float jx, jy, jz, cf, bailout2;
   int N;
   bool julia;
@@ -2102,6 +2104,8 @@ template <typename T, bool EFX = false>
 __device__ __forceinline__ bool secondary_step(const ParamsT<T> &p, const WaveBufs<T> &wb, SecondaryRay<T> &s,
                                                const T dist, const bool mi) {
   bool done = false;
+  // the factor is 1 until the ray ends, unless iteration fog absorbs along the march
+  const bool dark = EFX && s.sh < T(0);
   if (s.kind == 0) {
     if (p.softShadow) {
       T angle = (dist - s.thr) / s.r;
@@ -2112,20 +2116,20 @@ __device__ __forceinline__ bool secondary_step(const ParamsT<T> &p, const WaveBu
       if (soft < T(0)) soft = T(0);
       if (soft > s.maxSoft) s.maxSoft = soft;
     }
-    if (dist < s.thr || s.sh < T(0)) {
+    if (dist < s.thr || dark) {
       s.sh -= (s.end - s.r) / s.end;
       if (!p.penetrating) s.sh = T(0);
       if (s.sh < T(0)) s.sh = T(0);
       done = true;
     }
   } else if (!EFX || s.kind == 1) {
-    if (dist < s.thr || mi || s.sh < T(0)) {
+    if (dist < s.thr || mi || dark) {
       s.sh -= (s.end - s.r) / s.end;
       if (s.sh < T(0)) s.sh = T(0);
       done = true;
     }
   } else {
-    if (dist < s.thr || mi || s.sh < T(0)) {
+    if (dist < s.thr || mi || dark) {
       if (p.penetrating) {
         s.sh -= (s.end - s.r) / s.end;
         if (s.sh < T(0)) s.sh = T(0);

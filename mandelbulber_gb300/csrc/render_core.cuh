@@ -272,8 +272,6 @@ template <bool FULL>
 __device__ __forceinline__ double mandelbox_strict(const FractalT<double> &f, const V3<double> p, const int N,
                                                    int &Lout, Counters &cnt, const double scale) {
   const V3<double> c = f.juliaMode ? V3<double>{f.julia[0], f.julia[1], f.julia[2]}
-                       : f.constantFactor == 1.0   // the usual factor: three products less
-                                   ? p
                                    : V3<double>{__dmul_rn(p.x, f.constantFactor), __dmul_rn(p.y, f.constantFactor),
                                                 __dmul_rn(p.z, f.constantFactor)};
   int L;
@@ -396,13 +394,12 @@ __device__ __forceinline__ bool limit_box(const FractalT<T> &f, const V3<T> poin
 // CalculateDistance after the orbit (src/fractal.cpp:1291-1300, 1436-1445): the clamp at 0,
 // minN, interior mode, the iteration threshold and the limit box, on the orbit's distance
 // and end iteration Li. Shared by the generic and the lean orbits.
-// NONNEG: the distance is never negative (the strict orbit's), so the clamp falls away.
-template <typename T, bool NONNEG = false>
+template <typename T>
 __device__ __forceinline__ T distance_post(const FractalT<T> &f, T distance, const int Li, const int N, const int minN,
                                            const T detailSize, const bool normalMode, const T limitBoxDist,
                                            bool &maxIter) {
   maxIter = (Li == N);
-  if (!NONNEG && distance < T(0)) distance = T(0);
+  if (distance < T(0)) distance = T(0);
   if (Li < minN && distance < detailSize) distance = detailSize;
   if (!f.distPost) return distance;   // none of the three below: one uniform test per estimate
   if (f.interiorMode && !normalMode) {
@@ -447,12 +444,9 @@ __device__ __forceinline__ T calc_distance(const FractalT<T> &f, const V3<T> poi
       distance = compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
     }
   } else if constexpr (kStrictF64 && sizeof(T) == 8 && FORMULA == 8) {
-    if (f.boxStrict && box_strict_point(point.x, point.y, point.z)) {
-      distance = mandelbox_strict<FULL>(f, point, N, Li, cnt, fparam);
-      L = Li;
-      return distance_post<T, true>(f, distance, Li, N, minN, detailSize, normalMode, limitBoxDist, maxIter);
-    }
-    distance = compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
+    distance = f.boxStrict && box_strict_point(point.x, point.y, point.z)
+                   ? mandelbox_strict<FULL>(f, point, N, Li, cnt, fparam)
+                   : compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
   } else {
     distance = compute<T, FORMULA, 0>(f, point, N, Li, cnt, fparam);
   }

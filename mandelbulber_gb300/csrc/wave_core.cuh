@@ -2104,8 +2104,6 @@ template <typename T, bool EFX = false>
 __device__ __forceinline__ bool secondary_step(const ParamsT<T> &p, const WaveBufs<T> &wb, SecondaryRay<T> &s,
                                                const T dist, const bool mi) {
   bool done = false;
-  // the factor is 1 until the ray ends, unless iteration fog absorbs along the march
-  const bool dark = EFX && s.sh < T(0);
   if (s.kind == 0) {
     if (p.softShadow) {
       T angle = (dist - s.thr) / s.r;
@@ -2116,20 +2114,20 @@ __device__ __forceinline__ bool secondary_step(const ParamsT<T> &p, const WaveBu
       if (soft < T(0)) soft = T(0);
       if (soft > s.maxSoft) s.maxSoft = soft;
     }
-    if (dist < s.thr || dark) {
+    if (dist < s.thr || s.sh < T(0)) {
       s.sh -= (s.end - s.r) / s.end;
       if (!p.penetrating) s.sh = T(0);
       if (s.sh < T(0)) s.sh = T(0);
       done = true;
     }
   } else if (!EFX || s.kind == 1) {
-    if (dist < s.thr || mi || dark) {
+    if (dist < s.thr || mi || s.sh < T(0)) {
       s.sh -= (s.end - s.r) / s.end;
       if (s.sh < T(0)) s.sh = T(0);
       done = true;
     }
   } else {
-    if (dist < s.thr || mi || dark) {
+    if (dist < s.thr || mi || s.sh < T(0)) {
       if (p.penetrating) {
         s.sh -= (s.end - s.r) / s.end;
         if (s.sh < T(0)) s.sh = T(0);

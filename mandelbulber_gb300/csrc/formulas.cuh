@@ -114,7 +114,12 @@ __device__ __forceinline__ void tglad_step(const FractalT<T> &f, V3<T> &z, T &r,
 // One trig_optim Mandelbulb iteration (src/fractal.cpp:211-225).
 template <typename T>
 __device__ __forceinline__ void trig_optim_step(V3<T> &z, T &r, T &r_dz, const T p, const V3<T> constant) {
-  const T th0 = m_asin(z.z / r);
+  // the FP64 policy's quotient and root by integers, beside the FP64 pipe that asin, atan2, pow and
+  // sincos fill (the same bits): 192x192 deep zoom 111.3 -> 108.0 ms
+  T sz;
+  if constexpr (kStrictF64 && sizeof(T) == 8) sz = div_int(z.z, r);
+  else sz = z.z / r;
+  const T th0 = m_asin(sz);
   const T ph0 = m_atan2(z.y, z.x);
   T rp = m_pow(r, p - T(1));
   const T th = th0 * p;
@@ -125,7 +130,8 @@ __device__ __forceinline__ void trig_optim_step(V3<T> &z, T &r, T &r_dz, const T
   r_dz = rp * r_dz * p + T(1);
   rp *= r;
   z = V3<T>{cth * cph, cth * sph, sth} * rp + constant;
-  r = orbit_length(z);
+  if constexpr (kStrictF64 && sizeof(T) == 8) r = sqrt_int(dot3(z, z));
+  else r = orbit_length(z);
 }
 
 // Reflection across the closest cutting plane that meets the segment y + a * l, a in (0, 1]

@@ -374,7 +374,8 @@ static void fill_fractal(const mbgb_scene &s, FractalT<T> &f) {
   f.sphFixed = (T)s.foldingSphericalFixed;
   f.sphMin = (T)s.foldingSphericalMin;
   f.mbScale = (T)s.mboxScale;
-  f.mbFoldLimit = (T)s.mboxFoldingLimit;
+  // (the strict and lean orbits compare the limit's bits: -0 folds as 0 does)
+  f.mbFoldLimit = s.mboxFoldingLimit == 0.0 ? T(0) : (T)s.mboxFoldingLimit;
   f.mbFoldValue = (T)s.mboxFoldingValue;
   f.mbMinR = (T)s.mboxFoldingSphericalMin;
   f.mbFixedR = (T)s.mboxFoldingSphericalFixed;

@@ -273,8 +273,8 @@ static int distance_kernel_formula(const mbgb_scene &s) {
 }
 
 // The lean FP32 Mandelbox orbit applies: formula 8 without rotations, offset, pre-folds,
-// julia or primitive objects, fold value = 2 x fold limit, and min radius <= fixed radius (so
-// that the sphere fold is a clamp). The limit box, interior mode and the iteration threshold
+// julia or primitive objects, fold value = 2 x fold limit, and min radius <= fixed radius in
+// magnitude too, since the fold takes their squares (so that the sphere fold is a clamp). The limit box, interior mode and the iteration threshold
 // only test the point before the orbit or post-process its result (limit_box, distance_post),
 // which every lean path applies.
 static bool fast_mandelbox(const mbgb_scene &s) {
@@ -282,7 +282,8 @@ static bool fast_mandelbox(const mbgb_scene &s) {
          !s.tgladFoldingMode && !s.sphericalFoldingMode && !s.ifsFoldingMode && !uses_primitives(s) &&
          s.mboxOffset[0] == 0.0 && s.mboxOffset[1] == 0.0 && s.mboxOffset[2] == 0.0 &&
          s.mboxFoldingValue == 2.0 * s.mboxFoldingLimit &&
-         s.mboxFoldingSphericalMin <= s.mboxFoldingSphericalFixed;
+         s.mboxFoldingSphericalMin <= s.mboxFoldingSphericalFixed &&
+         fabs(s.mboxFoldingSphericalMin) <= fabs(s.mboxFoldingSphericalFixed);
 }
 
 // The power-8 Mandelbulb orbit without transcendentals applies (formula 2, power 8,

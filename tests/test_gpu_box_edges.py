@@ -32,3 +32,16 @@ def test_fold_limit_of_negative_zero_folds(gpu_ctx, oracle, value):
         got, want = gpu_ctx.render(sc, **o), gpu_ctx.render(plus, **o)
         for k in LAYERS:
             np.testing.assert_array_equal(getattr(got, k), getattr(want, k), err_msg=f"{o} layer {k}")
+
+
+@pytest.mark.parametrize("radius", [2.0, 1.2])
+def test_min_radius_beyond_the_fixed_one_has_no_sign(gpu_ctx, oracle, radius):
+    """The sphere fold squares its radii: a min radius of -2 is the frame of 2, whose fold is no
+    clamp, so the lean FP32 orbit applies to neither."""
+    minus, plus = (W.workload("mandelbox_1080p", 96, 54, mandelbox_folding_min_radius=r) for r in (-radius, radius))
+    ref, _ = oracle_lib.render(oracle, minus)
+    for o in ({}, {"polish_all": True}, {"precision": mb.PREC_FP64}):
+        got, want = gpu_ctx.render(minus, **o), gpu_ctx.render(plus, **o)
+        for k in LAYERS:
+            np.testing.assert_array_equal(getattr(got, k), getattr(want, k), err_msg=f"{o} layer {k}")
+        np.testing.assert_array_equal(got.hit, ref.hit)

@@ -1229,6 +1229,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const __grid_constant__ Par
       step = (double)wb.step[gp];
       detail = (double)wb.detail[gp];
       left = wb.bis_left[gp];
+      iters = wb.iters[gp];   // an estimate that ends at the limit box keeps the last orbit's
       thr = thr_of(scan);
       dist = polish_distance<FORMULA, FAST>(fd, point_of(scan), detail, iters, mi, cnt, fparam);
       cnt.steps++;
@@ -1266,7 +1267,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const __grid_constant__ Par
           else ns += ss;
         }
         const double nt = thr_of(ns);
-        int nl = 0;
+        int nl = -1;   // (no orbit ran: the limit box)
         Counters c1{0, 0, 0, 0};
         double nd = 0.0;
         if (depth < kPolishLevels && it + depth < n)
@@ -1278,7 +1279,8 @@ __global__ void __launch_bounds__(128) polish_kernel(const __grid_constant__ Par
           sc = __shfl_sync(0xffffffffu, ns, src);
           th = __shfl_sync(0xffffffffu, nt, src);
           di = __shfl_sync(0xffffffffu, nd, src);
-          li = __shfl_sync(0xffffffffu, nl, src);
+          const int ran = __shfl_sync(0xffffffffu, nl, src);
+          li = ran >= 0 ? ran : li;
           ob = __shfl_sync(0xffffffffu, c1.objectOut, src);
           if ((int)lane == src) {
             cnt.orbit += c1.orbit;

@@ -310,6 +310,33 @@ __device__ __forceinline__ F2 f2_atan(const F2 t, const F2 d) {
   return neg ? F2{-r.h, -r.l} : r;
 }
 
+// Error of the sum of a pixel's `quality` angles in pairs of floats.
+__host__ __device__ inline double ssao_sum_error(const int quality) { return 1e-12 * quality; }
+
+// A sample's slope from a pixel at plane position (ax, ay) of depth zs 2^20, aa = |ax| + |ay|:
+// lo <= slope <= up, infinite where FP32 does not tell (ssao_flat_kernel).
+constexpr float kSsaoScale = 9.5367431640625e-07f;   // 2^-20
+__device__ __forceinline__ void ssao_bracket(const SsaoSample &s, const float ax, const float ay, const float aa,
+                                             const float zs, const float z2, float &lo, float &up) {
+  const float t = fmaf(-z2, kSsaoScale, zs), cc = __uint_as_float(s.cc);
+  const float dx = fmaf(ax + s.cx, -t, s.cx * zs), dy = fmaf(ay + s.cy, -t, s.cy * zs);
+  const float inv = rsqrtf(fmaf(dx, dx, dy * dy)), slope = t * inv;
+  const float e = fmaf(aa + cc, fabsf(t), cc * zs);
+  const float rel = fmaf(e, 4.8e-7f * inv, 4e-6f), d = 1.15f * fabsf(slope) * rel;
+  const bool known = rel < 0.1f && fabsf(slope) < 1e30f;   // (false for NaN)
+  lo = known ? slope - d : -INFINITY;
+  up = known ? slope + d : INFINITY;
+}
+
+// The depth from which a pixel's slopes are bracketed. Below it the squares of plane distances
+// d = |c| z 2^-20 and less are subnormal floats, whose roundings (2 x 2^-150, so 7e-46 / d^2 of 1 / d)
+// rel does not hold: known brackets have d > 4.8e-6 E, E = |c| z 2^-20, and leave 0.04 rel >=
+// 0.04 x 4.8e-7 E / d, which covers them for E >= 9e-17. A sample's offset c is |persp| aspect /
+// (2 quality^2) at least; the limit keeps E at twice that.
+inline float ssao_least_depth(const int quality, const double persp, const double aspect) {
+  return (float)std::max(1e-6, 4e-10 * quality * quality / (fabs(persp) * aspect));
+}
+
 // The flat horizon search's inputs and outputs. `open` receives the pixels that the FP32 pass
 // leaves to ssao_exact_kernel, `opens` their number.
 struct SsaoArgs {
@@ -318,6 +345,7 @@ struct SsaoArgs {
   const uint8_t *colour;
   uint16_t *image16;
   int width, height, quality;
+  float zMin;                  // ssao_least_depth
   double persp, intensity;
   const SsaoSample *samples;   // [quality][quality - 1]
   const SsaoOffset *offsets;
@@ -373,18 +401,8 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
       const F2 axp = f2_of((mbgb::dev::div_int((double)x, w) - 0.5) * aspect * g.persp);
       const F2 ayp = f2_of((mbgb::dev::div_int((double)y, h) - 0.5) * g.persp);
       const float aa = fabsf(axp.h) + fabsf(ayp.h);
-      bool open = !(zf > 1e-6f && zf < 1e6f && aa < 1e3f);   // outside the forms' range
-      const float zs = zf * 9.5367431640625e-07f;            // 2^-20
-      auto bracket = [&](const SsaoSample &s, const float z2, float &lo, float &up) {
-        const float t = fmaf(-z2, 9.5367431640625e-07f, zs), cc = __uint_as_float(s.cc);
-        const float dx = fmaf(axp.h + s.cx, -t, s.cx * zs), dy = fmaf(ayp.h + s.cy, -t, s.cy * zs);
-        const float inv = rsqrtf(fmaf(dx, dx, dy * dy)), slope = t * inv;
-        const float e = fmaf(aa + cc, fabsf(t), cc * zs);
-        const float rel = fmaf(e, 4.8e-7f * inv, 4e-6f), d = 1.15f * fabsf(slope) * rel;
-        const bool known = rel < 0.1f && fabsf(slope) < 1e30f;   // (false for NaN)
-        lo = known ? slope - d : -INFINITY;
-        up = known ? slope + d : INFINITY;
-      };
+      bool open = !(zf > g.zMin && zf < 1e6f && aa < 1e3f);   // outside the forms' range
+      const float zs = zf * kSsaoScale;
       // a sample's angle and the bound of its error
       auto angle = [&](const SsaoSample &s, const int at, const float z2f, float &err) {
         // the background's depth is 1e20: the slope does not change with the scale
@@ -413,7 +431,7 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
           int at;
           const bool ok = ssao_sample(g, s, first + r, x, y, at);
           float lo, up;
-          bracket(s, g.zbuf[at], lo, up);
+          ssao_bracket(s, axp.h, ayp.h, aa, zs, g.zbuf[at], lo, up);
           lo = ok ? lo : -INFINITY;
           up = ok ? up : -INFINITY;
           const bool better = lo > bestLo;
@@ -435,7 +453,7 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
             if (!ssao_sample(g, s, first + r, x, y, at)) continue;
             const float z2 = g.zbuf[at];
             float lo, up, er;
-            bracket(s, z2, lo, up);
+            ssao_bracket(s, axp.h, ayp.h, aa, zs, z2, lo, up);
             if (!(up >= bestLo)) continue;
             const F2 t = angle(s, first + r, z2, er);
             err = fmaxf(err, er);
@@ -448,7 +466,7 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
       // the mean of 1/2 - angle / pi, and its error with that of the summation
       const double per = 1.0 / (kPi * g.quality);
       total = 0.5 - ((double)sum.h + (double)sum.l) * per;
-      error = ((double)errSum * 1.001 + 1e-12 * g.quality) * per;
+      error = ((double)errSum * 1.001 + ssao_sum_error(g.quality)) * per;
       if (open || !(error < 1e-3)) error = 2.0;
     }
     const double op = (double)g.opacity[i] / 65535.0;
@@ -601,6 +619,7 @@ mbgb_status ssao_device(const mbgb_scene &scene, const mbgb_image &layers, uint1
     } else {
       const SsaoScratch m = ssao_scratch(tables, q, n);
       const SsaoArgs g{layers.zbuffer, layers.opacity, layers.colour, image16, layers.width, layers.height, q,
+                       ssao_least_depth(q, scene.persp, (double)layers.width / layers.height),
                        scene.persp, scene.globalIlum, m.samples, m.offsets, m.opens, m.open};
       e = cudaMemsetAsync(m.opens, 0, sizeof(uint32_t), s);
       ssao_table_kernel<<<grid_for((int64_t)q * (q - 1), block), block, 0, s>>>(m.samples, m.offsets, layers.width,

@@ -310,8 +310,10 @@ __device__ __forceinline__ F2 f2_atan(const F2 t, const F2 d) {
   return neg ? F2{-r.h, -r.l} : r;
 }
 
-// Error of the sum of a pixel's `quality` angles in pairs of floats.
-__host__ __device__ inline double ssao_sum_error(const int quality) { return 1e-12 * quality; }
+// Error of the sum of a pixel's `quality` angles in pairs of floats: f2_add's three roundings of low
+// parts are 2^-48 of its operands each, so the addition of angle i errs by 3 x 2^-48 (i + 1) pi / 2,
+// 8.4e-15 q^2 + 2.5e-14 q in all.
+__host__ __device__ inline double ssao_sum_error(const int quality) { return (1e-12 + 1e-14 * quality) * quality; }
 
 // A sample's slope from a pixel at plane position (ax, ay) of depth zs 2^20, aa = |ax| + |ay|:
 // lo <= slope <= up, infinite where FP32 does not tell (ssao_flat_kernel).

@@ -36,6 +36,20 @@ __global__ void bracket_kernel(const int n, const float *z, const float *z2, con
     outside[i] = !((double)lo <= slope && slope <= (double)up);
   }
 }
+// the sum of q equal angles in pairs of floats against q c, in units of its bound
+__global__ void sum_kernel(const int n, const double *c, const int quality, double *ratio) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const F2 a = f2_of(c[i]);
+    F2 sum{0.0f, 0.0f};
+    for (int k = 0; k < quality; k++) sum = f2_add(sum, a);
+    const double v = (double)a.h + (double)a.l;
+    ratio[i] = fabs(((double)sum.h + (double)sum.l) - quality * v) / ssao_sum_error(quality);
+  }
+}
+}
+extern "C" int sums(int n, const double *c, int quality, double *ratio) {
+  sum_kernel<<<256, 128>>>(n, c, quality, ratio);
+  return (int)cudaDeviceSynchronize();
 }
 extern "C" float least_depth(int quality, double persp, double aspect) { return ssao_least_depth(quality, persp, aspect); }
 extern "C" int brackets(int n, const float *z, const float *z2, const double *ax, const double *ay, const double *cx,
@@ -103,6 +117,16 @@ def test_brackets_hold_the_slope(lib, quality, persp):
     t, p = _cuda(z, z2, ax, ay, rr * np.cos(a), rr * np.sin(a), outside)
     assert lib.brackets(n, *p) == 0
     assert int(t[6].sum()) == 0
+
+
+@pytest.mark.parametrize("quality", [1, 2, 20, 333, 1000])
+def test_angle_sum_stays_in_its_bound(lib, quality):
+    """Equal angles, whose roundings add up, over the angles' whole range."""
+    n = 400000
+    c = np.random.default_rng(quality).uniform(-np.pi / 2, np.pi / 2, n)
+    t, p = _cuda(c, np.zeros(n))
+    assert lib.sums(n, p[0], quality, p[1]) == 0
+    assert float(t[1].max()) <= 1.0
 
 
 def _depth(kind, w, h, rng):

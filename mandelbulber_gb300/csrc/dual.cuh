@@ -327,15 +327,11 @@ __device__ __forceinline__ bool escapes(const FractalT<T> &f, const V3<T> P, con
 // reference's binary refinement has put it inside the window (0.99 thr, thr)). Returns
 // false (and leaves t) when the level set is not reached: a grazing ray (F_t >= 0), a
 // flat estimate (orbit not escaping, minN clamp), or no convergence in 16 steps.
-// `bounded`: the FP32 refinement met an orbit that did not escape. Such a hit usually fails here
-// for the same reason after N iterations of the pipe-bound libm orbit, and its chain bounds the
-// stage, so the orbit is first run without tangents. Eight 256x256 frames 6.24 -> 5.91 ms.
 template <int FORMULA>
 __device__ __forceinline__ bool level_set_hit(const FractalT<double> &f, const V3<double> o, const V3<double> d,
                                               const double k, const double thrConst, double &t, int &iters,
-                                              const double fparam, const bool bounded) {
+                                              const double fparam) {
   double tt = t;
-  if (bounded && !escapes<double, FORMULA>(f, o + d * tt, f.N, fparam)) return false;
   for (int it = 0; it < 16; it++) {
     int L;
     const Dual<double, 1> de = de_along<double, FORMULA>(f, o + d * tt, d, f.N, L, fparam);
@@ -365,14 +361,13 @@ __device__ __forceinline__ bool level_set_hit(const FractalT<double> &f, const V
 template <int FORMULA>
 __device__ __forceinline__ bool level_set_hit_f32(const FractalT<float> &f, const V3<float> o, const V3<float> d,
                                                   const float k, const float thrConst, float &t, int &iters,
-                                                  const float fparam, bool &bounded) {
+                                                  const float fparam) {
   float tt = t;
   const float lenD = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
   for (int it = 0; it < 16; it++) {
     int L;
     const Dual<float, 1> de = de_along<float, FORMULA>(f, o + d * tt, d, f.N, L, fparam);
     const float thr = k > 0.0f ? tt * k : thrConst;
-    if (L == f.N) bounded = it == 0;
     if (L == f.N || L < f.minN || !isfinite(de.v) || !isfinite(de.d[0])) return false;
     const float F = de.v - thr;
     if (fabsf(F) <= 2e-5f * thr) {

@@ -26,6 +26,7 @@
 // of the ballot).
 #pragma once
 
+#include "job_share.cuh"
 #include "dual.cuh"
 #include "render_core.cuh"
 #include "wave_launch.h"
@@ -352,23 +353,12 @@ __device__ __forceinline__ unsigned int claim_jobs(unsigned int *counter, const 
   return base + (unsigned int)__popc(mask & ((1u << lane) - 1u));
 }
 
-// How a stage's warps share its jobs. A stage with fewer jobs than lanes hands each warp only as
-// many as let `wb.spread` warps take part, and only the first warps take any (blocks start one
-// per SM, so those spread evenly over the SMs and their sub-partitions). `lanes`: the lanes of a
-// warp that take jobs; `warps`: the warps that do.
-struct JobShare {
-  unsigned int lanes, warps, refill;
-  bool idle;   // this lane takes none
-};
+// This launch's share of a stage's `jobs`, and whether this lane takes any.
 template <typename T>
-__device__ __forceinline__ JobShare job_share(const WaveBufs<T> &wb, const unsigned int jobs) {
-  JobShare s;
-  const unsigned int spread = (unsigned int)wb.spread;
-  s.lanes = jobs >= 32u * spread ? 32u : max(1u, (jobs + spread - 1) / spread);
-  s.warps = (jobs + s.lanes - 1) / s.lanes;
-  s.refill = min((unsigned int)wb.refill_min, max(1u, s.lanes / 4));
-  const unsigned int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  s.idle = (threadIdx.x & 31u) >= s.lanes || warp >= s.warps;
+__device__ __forceinline__ JobShare job_share(const WaveBufs<T> &wb, const unsigned int jobs, bool &idle) {
+  const unsigned int wpb = blockDim.x >> 5;
+  const JobShare s = job_share(jobs, (unsigned int)wb.spread, gridDim.x * wpb, (unsigned int)wb.refill_min);
+  idle = (threadIdx.x & 31u) >= s.lanes || blockIdx.x * wpb + (threadIdx.x >> 5) >= s.warps;
   return s;
 }
 
@@ -918,8 +908,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : FAST ? 8 : 6) primar
   unsigned int *jobCounter = io.overflow_pass ? (wb.ctl + 4) : (wb.ctl + 0);
 
   // per-lane ray state
-  const JobShare share = job_share(wb, nJobs);
-  bool active = false, exhausted = share.idle;
+  bool active = false, exhausted;
+  const JobShare share = job_share(wb, nJobs, exhausted);
   int64_t gp = 0;   // pixel of the batch
   int64_t ri = 0;   // ray: depth * npix_frame + gp
   int phase = 0, i = 0, buffCount = 0, iters = 0, bis = 0;
@@ -2248,7 +2238,8 @@ __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const Fr
   unsigned int hitCalls = 0;
   LeanOrbit<FORMULA> orb(p.f);
   SecondaryRay<float> s{};
-  bool active = false, exhausted = job_share(wb, njobs).idle, orbiting = false;
+  bool active = false, exhausted, orbiting = false;
+  job_share(wb, njobs, exhausted);
   float odist = 0.0f;
   for (;;) {
     // lanes whose orbit ended: the distance estimate's clamps, then the ray's step
@@ -2483,8 +2474,8 @@ __global__ void __launch_bounds__(128) secondary_kernel(const __grid_constant__ 
   const SecondaryJobs jn = secondary_jobs<T, EFX>(p, wb, nh);
   const unsigned int njobs = jn.nShadow + jn.nAO + jn.nAux + (unsigned int)wb.sample_nres * jn.nSamples;
   Counters cnt{0, 0, 0, 0};
-  const JobShare share = job_share(wb, njobs);
-  bool active = false, exhausted = share.idle;
+  bool active = false, exhausted;
+  const JobShare share = job_share(wb, njobs, exhausted);
   SecondaryRay<T> s{};
   for (;;) {
     // a warp claims new jobs once refill_min of its lanes are idle, or when none is busy

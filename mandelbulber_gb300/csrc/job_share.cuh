@@ -7,7 +7,7 @@ namespace mbgb {
 namespace dev {
 
 // `lanes`: the lanes of a warp that take jobs; `warps`: the launch's first warps, which do;
-// `refill`: idle lanes before a warp claims again.
+// `refill`: idle lanes before a warp claims again, a quarter of its lanes at most unless it has all.
 struct JobShare {
   unsigned int lanes, warps, refill;
 };
@@ -25,7 +25,7 @@ __host__ __device__ __forceinline__ JobShare job_share(const unsigned int jobs, 
   if (s.lanes < 1u) s.lanes = 1u;
   s.warps = (jobs + s.lanes - 1) / s.lanes;
   const unsigned int quarter = s.lanes / 4 > 1u ? s.lanes / 4 : 1u;
-  s.refill = refill_min < quarter ? refill_min : quarter;
+  s.refill = s.lanes == 32u || refill_min < quarter ? refill_min : quarter;
   return s;
 }
 

@@ -43,3 +43,10 @@ def test_every_job_finds_a_lane_where_there_are_enough(share, spread, launched):
         lanes, warps, _ = share(jobs, spread, launched)
         assert 1 <= lanes <= 32 and (warps - 1) * lanes < max(jobs, 1)
         assert lanes * min(warps, launched) >= min(jobs, 32 * launched), (jobs, lanes, warps)
+
+
+@pytest.mark.parametrize("refill", [1, 4, 8, 16, 32])
+def test_full_warps_claim_at_the_threshold_that_was_asked_for(share, refill):
+    assert share(2_000_000, 2432, 4864, refill) == (32, 62500, refill)
+    lanes, _, got = share(19200, 2432, 4864, refill)   # 160x120: eight lanes a warp
+    assert (lanes, got) == (8, min(refill, 2))

@@ -400,10 +400,14 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
     const float zf = g.zbuf[i];
     double total = 0.0, error = 0.0;
     if ((double)zf < 1e19) {
+      if (!(zf > g.zMin && zf < 1e6f && g.intensity >= 0.0)) {   // outside the forms' range: no pass
+        g.open[atomicAdd(g.opens, 1u)] = (uint32_t)i;
+        continue;
+      }
       const F2 axp = f2_of((mbgb::dev::div_int((double)x, w) - 0.5) * aspect * g.persp);
       const F2 ayp = f2_of((mbgb::dev::div_int((double)y, h) - 0.5) * g.persp);
       const float aa = fabsf(axp.h) + fabsf(ayp.h);
-      bool open = !(zf > g.zMin && zf < 1e6f && aa < 1e3f);   // outside the forms' range
+      bool open = !(aa < 1e3f);
       const float zs = zf * kSsaoScale;
       // a sample's angle and the bound of its error
       auto angle = [&](const SsaoSample &s, const int at, const float z2f, float &err) {
@@ -475,7 +479,7 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
     const double gain = 65535.0 / 256.0 * g.intensity * (1.0 - op);
     const double lowT = fmax(total - error, 0.0), highT = fmax(total + error, 0.0);
     // (an error of 0 is the background's: its term is exactly 0)
-    bool settled = error == 0.0 || (error < 1.0 && g.intensity >= 0.0);
+    bool settled = error < 1.0;
     uint16_t out[3];
     for (int c = 0; c < 3; c++) {
       const uint16_t was = g.image16[3 * i + c];
@@ -493,25 +497,35 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
 }
 
 // The pixels that ssao_flat_kernel leaves open, every slope in double as ThreadSSAO forms it (the
-// values of ssao_kernel<double> bit for bit), one warp a pixel: a lane takes every 32nd direction,
-// and the directions' terms are summed in the reference's order.
+// values of ssao_kernel<double> bit for bit): a lane takes a direction (every 32nd of more than 32),
+// and the directions' terms are summed in the reference's order. A warp holds as many pixels as
+// leave a lane to each direction: with one each, a frame whose depths all lie below the FP32 forms'
+// range (a camera a millionth from the surface) took longer than ssao_kernel<double>, 1024x768 at
+// quality 4 / 6 / 10 / 20 6.7 / 8.5 / 12.1 / 21.8
+// against 1.33 / 2.84 / 7.7 / 30.4 ms, as it stands 0.88 / 2.13 / 5.9 / 20.8.
 __global__ void __launch_bounds__(128) ssao_exact_kernel(const __grid_constant__ SsaoArgs g) {
   using mbgb::dev::div_int;
   using mbgb::dev::sqrt_int;
   const uint32_t n = *g.opens;
   const double w = (double)g.width, h = (double)g.height, aspect = w / h;
   const int lane = threadIdx.x & 31, steps = g.quality - 1;
-  for (uint32_t k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < n; k += gridDim.x * (blockDim.x >> 5)) {
-    const int64_t i = g.open[k];
+  int lanes = 32;   // of a pixel
+  while (lanes / 2 >= g.quality) lanes /= 2;
+  const uint32_t per = 32u / lanes, own = (uint32_t)lane / lanes;
+  const int sub = lane & (lanes - 1);
+  const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t k0 = warp * per; k0 < n; k0 += warps * per) {
+    const bool valid = k0 + own < n;   // (else the warp's first pixel again, unwritten)
+    const int64_t i = g.open[valid ? k0 + own : k0];
     const int x = (int)(i % g.width), y = (int)(i / g.width);
     const double z = (double)g.zbuf[i];
     double ambient = 0.0;
     const double x2 = (div_int((double)x, w) - 0.5) * aspect * z * g.persp;
     const double y2 = (div_int((double)y, h) - 0.5) * z * g.persp;
-    for (int a0 = 0; a0 < g.quality; a0 += 32) {
+    for (int a0 = 0; a0 < g.quality; a0 += lanes) {
       double term = 0.0;
-      if (a0 + lane < g.quality) {
-        const int first = (a0 + lane) * steps;
+      if (a0 + sub < g.quality) {
+        const int first = (a0 + sub) * steps;
         double maxDiff = -1e50;
         for (int r = 0; r < steps; r++) {
           int at;
@@ -525,16 +539,17 @@ __global__ void __launch_bounds__(128) ssao_exact_kernel(const __grid_constant__
         }
         term = div_int(-atan(maxDiff), kPi) + 0.5;
       }
-      for (int l = 0; l < 32 && a0 + l < g.quality; l++) ambient += __shfl_sync(0xffffffffu, term, l);
+      for (int l = 0; l < lanes && a0 + l < g.quality; l++) ambient += __shfl_sync(0xffffffffu, term, l, lanes);
     }
     double total = ambient / (double)g.quality;
     if (total < 0.0) total = 0.0;
-    if (lane < 3) {
+    if (!valid) continue;
+    for (int c = sub; c < 3; c += lanes) {
       const double op = (double)g.opacity[i] / 65535.0;
-      double v = (double)g.image16[3 * i + lane] +
-                 65535.0 * (double)g.colour[3 * i + lane] / 256.0 * total * g.intensity * (1.0 - op);
+      double v = (double)g.image16[3 * i + c] +
+                 65535.0 * (double)g.colour[3 * i + c] / 256.0 * total * g.intensity * (1.0 - op);
       if (v > 65535.0) v = 65535.0;
-      g.image16[3 * i + lane] = (uint16_t)(unsigned short)v;
+      g.image16[3 * i + c] = (uint16_t)(unsigned short)v;
     }
   }
 }

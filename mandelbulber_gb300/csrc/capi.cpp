@@ -1135,9 +1135,10 @@ struct WaveLayout {
 // `auxN` auxiliary lights: hit normals, and with `auxShadows` one AuxShadow factor per light.
 // `sampleRes` > 0 (volumetric lights, iteration fog): the volumetric walk's samples (at most
 // one per pool record) with `sampleRes` results each; `iterFog`: the records' itersOut.
-// `jobs`: the primary jobs of the group, over which the hit list's compaction walks.
+// `jobs`: the primary jobs of the group, over which the hit list's compaction walks. `hitJobs`:
+// runs_hit_jobs, the shadow stage's values of each hit.
 static WaveLayout wave_layout(int64_t npixFrame, size_t ts, int aoN, bool needVol, int rays, int auxN,
-                              bool auxShadows, int sampleRes, bool iterFog, int64_t jobs) {
+                              bool auxShadows, int sampleRes, bool iterFog, int64_t jobs, bool hitJobs) {
   const int64_t npix = npixFrame * rays;
   WaveLayout w{};
   size_t off = 0;
@@ -1187,7 +1188,7 @@ static WaveLayout wave_layout(int64_t npixFrame, size_t ts, int aoN, bool needVo
   w.piters = take(iterFog && needVol ? (size_t)w.poolCap * kChunk * 4 : 0);
   w.segc = take(rays == 1 ? (size_t)((jobs + kHitSeg - 1) / kHitSeg) * kHitSegWarps * 4 : 0);
   w.hset = take(rays == 1 ? (size_t)npix * 8 * ts : 0);
-  w.colr = take(rays == 1 ? 5 * (size_t)npix * ts : 0);   // colour, normal (or its distances), fast AO
+  w.colr = take(hitJobs ? 5 * (size_t)npix * ts : 0);   // colour, normal (or its distances), fast AO
   w.total = off;
   return w;
 }
@@ -1201,6 +1202,15 @@ static int wave_occupancy(int formula, int block, int which) {
 // Largest number of pixels x (1 + ray-AO directions) one wavefront group indexes with
 // 32-bit pixel and job numbers.
 constexpr double kMaxGroupJobs = 4.0e9;
+
+// Whether a group's shadow stage runs the hits' colouring orbits and shading estimates too
+// (secondary_lean), up to five more jobs per hit: the lean FP32 Mandelbulb's plain variant with
+// orbit-granular refill.
+static bool runs_hit_jobs(const mbgb_scene &s, int prec, const LaunchCfg &cfg, int64_t npix, int aoN) {
+  return prec == 1 && fast_mandelbulb(s) && !s.limits_enabled && reflection_rays(s) == 1 && !uses_aux_lights(s) &&
+         !s.volumetricLightEnabledAny && !s.iterFogEnabled && !s.fakeLightsEnabled && !s.slowShading &&
+         cfg.orbitRefill > 0 && (double)npix * (6.0 + aoN) < kMaxGroupJobs;
+}
 
 // Enqueue the wavefront stages (wave_core.cuh) of one group: primary rays, FP64 polish
 // (FP32 policy), shadow/AO rays, composition. No host round trips.
@@ -1219,8 +1229,9 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
       scene.volumetricLightEnabledAny != 0 || scene.iterFogEnabled != 0 || scene.fakeLightsEnabled != 0;
   const int sampleRes =
       volLights ? kSampleShadows + (scene.iterFogEnabled ? aoN : 0) + (scene.fakeLightsEnabled ? 1 : 0) : 0;
+  const bool hitJobs = runs_hit_jobs(scene, prec, g.cfg, g.npix, aoN);
   const WaveLayout w = wave_layout(g.npix, sizeof(T), aoN, needVol, rays, auxN, scene.shadow != 0, sampleRes,
-                                   scene.iterFogEnabled != 0, g.jobs);
+                                   scene.iterFogEnabled != 0, g.jobs, hitJobs);
   char *base = (char *)c->wave[prec].ptr;
   WaveLaunch<T> L;
   WaveBufs<T> &wb = L.wb;
@@ -1336,10 +1347,6 @@ static mbgb_status enqueue_wave(mbgb_context *c, const mbgb_scene *scenes, const
   // as the device's launch sequence.
   const bool efx = rays > 1 || L.p.numberOfLights > 0 || L.p.volLightAny || L.p.iterFog || L.p.fakeLights;
   const bool secondaryJobs = scene.shadow != 0 || rayAO;
-  // the lean Mandelbulb's shadow stage runs the hits' colouring orbits and shading estimates too
-  // (secondary_lean), up to five more jobs per hit
-  const bool hitJobs = sizeof(T) == 4 && kf == 2 && L.fast && !efx && !L.p.slowShading && g.cfg.orbitRefill > 0 &&
-                       (double)g.npix * (6.0 + aoN) < kMaxGroupJobs;
   wb.colour = hitJobs ? (T *)(base + w.colr) : nullptr;
   wb.lean_normal = hitJobs ? wb.colour + g.npix : nullptr;
   wb.lean_ao = hitJobs && scene.global_ilumination && scene.fastGlobalIllumination ? wb.colour + 4 * g.npix : nullptr;
@@ -1811,16 +1818,17 @@ static mbgb_status render_frames(mbgb_context *c, const mbgb_scene *scenes, int 
     if (g.wave) {
       const bool rayAO = rep.global_ilumination && !rep.fastGlobalIllumination;
       const size_t ts = g.prec == 0 ? sizeof(double) : sizeof(float);
+      const int aoN = rayAO ? c->ao_count : 0;
       wave_bytes[g.prec] =
-          std::max(wave_bytes[g.prec], wave_layout(g.npix, ts, rayAO ? c->ao_count : 0, needVol, reflection_rays(rep),
+          std::max(wave_bytes[g.prec], wave_layout(g.npix, ts, aoN, needVol, reflection_rays(rep),
                                                    aux_light_count(rep), rep.shadow != 0,
                                                    (rep.volumetricLightEnabledAny || rep.iterFogEnabled ||
                                                     rep.fakeLightsEnabled)
-                                                       ? kSampleShadows +
-                                                             (rep.iterFogEnabled && rayAO ? c->ao_count : 0) +
+                                                       ? kSampleShadows + (rep.iterFogEnabled ? aoN : 0) +
                                                              (rep.fakeLightsEnabled ? 1 : 0)
                                                        : 0,
-                                                   rep.iterFogEnabled != 0, g.jobs)
+                                                   rep.iterFogEnabled != 0, g.jobs,
+                                                   runs_hit_jobs(rep, g.prec, g.cfg, g.npix, aoN))
                                            .total);
       g.cams_off = camsBytes;
       const size_t cs = g.prec == 0 ? sizeof(FrameCam<double>) : sizeof(FrameCam<float>);

@@ -2375,7 +2375,8 @@ extern "C" mbgb_status mbgb_ssao_device(mbgb_context *c, const mbgb_scene *scene
   if (scene->SSAOQuality > 1000) return set_error(MBGB_ERR_BAD_PARAM, "SSAO quality above 1000");
   std::lock_guard<std::mutex> lk(c->mu);
   MBGB_CUDA(cudaSetDevice(c->device));
-  MBGB_CUDA(c->ensure(c->post, std::max<size_t>(sizeof(int) * 65536, ssao_scratch_bytes(scene->SSAOQuality, (int64_t)layers->width * layers->height))));
+  const size_t scratch = ssao_scratch_bytes(*scene, layers->width, (int64_t)layers->width * layers->height);
+  MBGB_CUDA(c->ensure(c->post, std::max<size_t>(sizeof(int) * 65536, scratch)));
   return ssao_device(*scene, *layers, image16, c->post.ptr, c->stream);
 }
 

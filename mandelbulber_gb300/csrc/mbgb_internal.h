@@ -40,7 +40,9 @@ int ao_vectors_into(int quality, float *out, int max_vectors);
 // Post-processing on the device (post.cu): CompileImage into RGB16 and the SSAO pass.
 mbgb_status compile16_device(const mbgb_scene &scene, const float *image_float, int width, int height,
                              uint16_t *image16, int *gamma_dev, cudaStream_t s);
-size_t ssao_scratch_bytes(int quality, int64_t npix);   // device scratch of ssao_device
+// device scratch of ssao_device: of the flat kernel, of a scene's frame
+size_t ssao_scratch_bytes(int quality, int64_t npix);
+size_t ssao_scratch_bytes(const mbgb_scene &scene, int width, int64_t npix);
 mbgb_status ssao_device(const mbgb_scene &scene, const mbgb_image &layers, uint16_t *image16, void *tables,
                         cudaStream_t s);
 mbgb_status dof_device(const mbgb_scene &scene, const mbgb_image &layers, uint16_t *image16, uint32_t seed,

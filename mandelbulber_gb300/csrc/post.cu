@@ -587,7 +587,15 @@ mbgb_status compile16_device(const mbgb_scene &scene, const float *image_float, 
   return MBGB_OK;
 }
 
-// Scratch of ssao_device: cos and sin of the directions, their samples, the open pixels.
+// Whether ssao_flat_kernel takes a frame: the flat projection, offsets of at most 16 bits and pixel
+// indices of at most 31.
+static bool ssao_flat(const mbgb_scene &scene, int width, int64_t npix) {
+  return scene.perspectiveType != MBGB_PERSP_FISH_EYE && scene.perspectiveType != MBGB_PERSP_EQUIRECT &&
+         width <= 64000 && npix < (int64_t)1 << 31;
+}
+
+// Scratch of ssao_device: cos and sin of the directions, and for the flat kernel their samples and
+// the open pixels.
 struct SsaoScratch {
   SsaoSample *samples;
   SsaoOffset *offsets;
@@ -608,6 +616,10 @@ static SsaoScratch ssao_scratch(void *base, int quality, int64_t npix) {
   return m;
 }
 size_t ssao_scratch_bytes(int quality, int64_t npix) { return ssao_scratch(nullptr, quality, npix).bytes; }
+size_t ssao_scratch_bytes(const mbgb_scene &scene, int width, int64_t npix) {
+  return ssao_flat(scene, width, npix) ? ssao_scratch_bytes(scene.SSAOQuality, npix)
+                                       : sizeof(double) * 2 * (size_t)std::max(scene.SSAOQuality, 0);
+}
 
 // PostRendering_SSAO on the device, in double (the reference's arithmetic): the sample
 // positions x + r^2 s cos(a) land on the neighbouring pixel or not depending on the last
@@ -627,9 +639,7 @@ mbgb_status ssao_device(const mbgb_scene &scene, const mbgb_image &layers, uint1
   const double *cs = (const double *)tables, *sn = cs + q;
   cudaError_t e = cudaMemcpyAsync(tables, t.data(), sizeof(double) * 2 * q, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) {
-    // (offsets past 16 bits and pixel indices past 31 take the general kernel too)
-    if (scene.perspectiveType == MBGB_PERSP_FISH_EYE || scene.perspectiveType == MBGB_PERSP_EQUIRECT ||
-        layers.width > 64000 || n >= (int64_t)1 << 31) {
+    if (!ssao_flat(scene, layers.width, n)) {
       ssao_kernel<double><<<grid_for(n, block), block, 0, s>>>(
           layers.zbuffer, layers.opacity, layers.colour, image16, layers.width, layers.height, scene.persp, q,
           scene.perspectiveType, scene.globalIlum, cs, sn);

@@ -1,5 +1,7 @@
 """Device memory that a context takes for a call (needs a GPU): buffers that only some scenes read are
 held by those alone."""
+import ctypes
+
 import pytest
 
 import mandelbulber_gb300 as mb
@@ -38,3 +40,27 @@ def test_hit_values_are_held_where_the_shadow_stage_writes_them(gpu_ctx):
     assert with_jobs - frame(formula=8) > values - 4 * MIB
     # FP64: every array at most twice as wide, without the values
     assert frame(precision=mb.PREC_FP64) < 2 * (with_jobs - values) + 4 * MIB
+
+
+def test_ssao_of_other_projections_holds_its_directions_alone(gpu_ctx):
+    """The flat kernel's samples (48 bytes x quality (quality - 1)) and open list (4 bytes a pixel):
+    fish eye and equirectangular frames run ssao_kernel<double>, which reads neither."""
+    import torch
+    w, h, quality = 64, 48, 1000
+    t = [torch.zeros((h, w), device="cuda") + 2.0, torch.zeros((h, w), dtype=torch.int16, device="cuda"),
+         torch.zeros((h, w, 3), dtype=torch.uint8, device="cuda"), torch.zeros((h, w, 3), dtype=torch.int16, device="cuda")]
+    t[0][:] = 1e20   # background: no search
+    p = [ctypes.c_void_p(v.data_ptr()) for v in t]
+    layers = mb.mbgb_image(w, h, None, p[0], None, p[1], p[2], None, None, None)
+
+    def call(ptype):
+        sc = W.workload("mandelbulb_640x480", w, h, post_SSAO_quality=quality)
+        sc.SSAOQuality, sc.perspectiveType = quality, ptype
+
+        def run(ctx):
+            assert mb.library().mbgb_ssao_device(ctx._h, ctypes.byref(sc), ctypes.byref(layers), t[3].data_ptr()) == 0
+        run(gpu_ctx)
+        return _held(run)
+    flat = call(0)
+    for ptype in (1, 2):
+        assert flat - call(ptype) > 48 * quality * (quality - 1) - 4 * MIB

@@ -1388,6 +1388,24 @@ __global__ void __launch_bounds__(128) level_set_kernel(const __grid_constant__ 
   if (missed) atomicAdd(wb.ctl + 7, missed);
 }
 
+// Sample i of the lean Mandelbulb's fast AO, its term and the factor of the terms' sum: rounded as
+// written here, since the shadow stage (shade_step) and the composition (wave_fast_ao, without
+// orbit-granular refill) form the same pixels.
+__device__ __forceinline__ V3<float> fast_ao_point(const V3<float> point, const V3<float> normal, const int i,
+                                                   const float thr) {
+  const float scan = __fmul_rn(float(i * i), thr);
+  return V3<float>{fmaf(normal.x, scan, point.x), fmaf(normal.y, scan, point.y), fmaf(normal.z, scan, point.z)};
+}
+__device__ __forceinline__ float fast_ao_term(const int i, const float thr, const float tune, const float dist) {
+  // 2^-i
+  const float w = i < 127 ? __uint_as_float((uint32_t)(127 - i) << 23) : i == 127 ? 5.877471754111438e-39f : 0.0f;
+  return __fdiv_rn(__fmul_rn(w, fmaf(float(i * i), thr, -__fmul_rn(tune, dist))), thr);
+}
+__device__ __forceinline__ float fast_ao_value(const float sum) {
+  const float ao = __fsub_rn(1.0f, __fmul_rn(0.2f, sum));
+  return ao < 0.0f ? 0.0f : ao;
+}
+
 // FastAmbientOcclusion2 (src/shaders.cpp:585-605) on the stage's orbit: q^2 - 1 DE samples
 // along the normal at i^2 x the threshold, weighted 2^-i.
 template <typename T, int FORMULA, bool FAST>
@@ -1396,14 +1414,21 @@ __device__ __forceinline__ T wave_fast_ao(const ParamsT<T> &p, const V3<T> point
   T aoTemp = T(0);
   const int q2 = p.aoQuality * p.aoQuality;
   for (int i = 1; i < q2; i++) {
-    const T scan = T(i * i) * dist_thresh;
-    const V3<T> pt = point + normal * scan;
     int L;
     bool mi;
+    if constexpr (FAST && FORMULA == 2 && sizeof(T) == 4) {
+      const float dist = wave_distance<T, FORMULA, FAST>(p.f, fast_ao_point(point, normal, i, dist_thresh), detail, p.f.N,
+                                                         p.f.minN, false, L, mi, cnt, fparam);
+      aoTemp = __fadd_rn(aoTemp, fast_ao_term(i, dist_thresh, p.fastAoTune, dist));
+      continue;
+    }
+    const T scan = T(i * i) * dist_thresh;
+    const V3<T> pt = point + normal * scan;
     const T dist = wave_distance<T, FORMULA, FAST>(p.f, pt, detail, p.f.N, p.f.minN, false, L, mi, cnt, fparam);
     // 1.0 / pow(2.0, i) is exact for integral i
     aoTemp += T(1) / T(ldexp(1.0, i)) * (scan - p.fastAoTune * dist) / dist_thresh;
   }
+  if constexpr (FAST && FORMULA == 2 && sizeof(T) == 4) return fast_ao_value(aoTemp);
   T ao = T(1) - T(0.2) * aoTemp;
   if (ao < T(0)) ao = T(0);
   return ao;
@@ -2157,9 +2182,7 @@ __device__ __forceinline__ V3<float> shade_point(const ParamsT<float> &p, const 
   if (s.j == 1) return V3<float>{s.point.x + s.r, s.point.y + 0.0f, s.point.z + 0.0f};
   if (s.j == 2) return V3<float>{s.point.x + 0.0f, s.point.y + s.r, s.point.z + 0.0f};
   if (s.j == 3) return V3<float>{s.point.x + 0.0f, s.point.y + 0.0f, s.point.z + s.r};
-  const int i = (int)s.j - 3;
-  const float scan = __fmul_rn(float(i * i), s.thr);
-  return V3<float>{fmaf(s.dir.x, scan, s.point.x), fmaf(s.dir.y, scan, s.point.y), fmaf(s.dir.z, scan, s.point.z)};
+  return fast_ao_point(s.point, s.dir, (int)s.j - 3, s.thr);
 }
 __device__ __forceinline__ void shade_begin(const ParamsT<float> &p, const WaveBufs<float> &wb,
                                             const FrameCam<float> *__restrict__ cams, const int ncams,
@@ -2195,19 +2218,14 @@ __device__ __forceinline__ bool shade_step(const ParamsT<float> &p, const WaveBu
     s.dir = n;
     s.sh = 0.0f;
   } else {
-    const int i = (int)s.j - 3;
-    // the roundings of wave_fast_ao as it compiles: i^2 thr fused into the difference
-    const float w = i < 127 ? __uint_as_float((uint32_t)(127 - i) << 23) : i == 127 ? 5.877471754111438e-39f : 0.0f;
-    s.sh += __fdiv_rn(__fmul_rn(w, fmaf(float(i * i), s.thr, -__fmul_rn(p.fastAoTune, d))), s.thr);
+    s.sh = __fadd_rn(s.sh, fast_ao_term((int)s.j - 3, s.thr, p.fastAoTune, d));
   }
   s.j++;
   if (s.j < 4) return false;
   const unsigned int last = (p.ao && p.fastAO) ? 3u + (unsigned int)(p.aoQuality * p.aoQuality) : 4u;
   if (s.j < last) return false;
   if (p.ao && p.fastAO) {
-    float ao = __fsub_rn(1.0f, __fmul_rn(0.2f, s.sh));
-    if (ao < 0.0f) ao = 0.0f;
-    wb.lean_ao[s.gp] = ao;
+    wb.lean_ao[s.gp] = fast_ao_value(s.sh);
   }
   return true;
 }

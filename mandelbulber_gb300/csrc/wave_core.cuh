@@ -353,13 +353,11 @@ __device__ __forceinline__ unsigned int claim_jobs(unsigned int *counter, const 
   return base + (unsigned int)__popc(mask & ((1u << lane) - 1u));
 }
 
-// This launch's share of a stage's `jobs`, and whether this lane takes any.
+// This lane's share of a stage's `jobs`.
 template <typename T>
-__device__ __forceinline__ JobShare job_share(const WaveBufs<T> &wb, const unsigned int jobs, bool &idle) {
-  const unsigned int wpb = blockDim.x >> 5;
-  const JobShare s = job_share(jobs, (unsigned int)wb.spread, gridDim.x * wpb, (unsigned int)wb.refill_min);
-  idle = (threadIdx.x & 31u) >= s.lanes || blockIdx.x * wpb + (threadIdx.x >> 5) >= s.warps;
-  return s;
+__device__ __forceinline__ JobShare job_share(const WaveBufs<T> &wb, const unsigned int jobs) {
+  return job_share(jobs, (unsigned int)wb.spread, (unsigned int)wb.refill_min,
+                   blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31u);
 }
 
 // One pooled step record: dist, thr, step in a 16-byte (float) or 32-byte (double) slot.
@@ -908,8 +906,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : FAST ? 8 : 6) primar
   unsigned int *jobCounter = io.overflow_pass ? (wb.ctl + 4) : (wb.ctl + 0);
 
   // per-lane ray state
-  bool active = false, exhausted;
-  const JobShare share = job_share(wb, nJobs, exhausted);
+  const JobShare share = job_share(wb, nJobs);
+  bool active = false, exhausted = share.idle;
   int64_t gp = 0;   // pixel of the batch
   int64_t ri = 0;   // ray: depth * npix_frame + gp
   int phase = 0, i = 0, buffCount = 0, iters = 0, bis = 0;
@@ -2256,8 +2254,7 @@ __device__ __forceinline__ void secondary_lean(const ParamsT<float> &p, const Fr
   unsigned int hitCalls = 0;
   LeanOrbit<FORMULA> orb(p.f);
   SecondaryRay<float> s{};
-  bool active = false, exhausted, orbiting = false;
-  job_share(wb, njobs, exhausted);
+  bool active = false, exhausted = job_share(wb, njobs).idle, orbiting = false;
   float odist = 0.0f;
   for (;;) {
     // lanes whose orbit ended: the distance estimate's clamps, then the ray's step
@@ -2492,8 +2489,8 @@ __global__ void __launch_bounds__(128) secondary_kernel(const __grid_constant__ 
   const SecondaryJobs jn = secondary_jobs<T, EFX>(p, wb, nh);
   const unsigned int njobs = jn.nShadow + jn.nAO + jn.nAux + (unsigned int)wb.sample_nres * jn.nSamples;
   Counters cnt{0, 0, 0, 0};
-  bool active = false, exhausted;
-  const JobShare share = job_share(wb, njobs, exhausted);
+  const JobShare share = job_share(wb, njobs);
+  bool active = false, exhausted = share.idle;
   SecondaryRay<T> s{};
   for (;;) {
     // a warp claims new jobs once refill_min of its lanes are idle, or when none is busy

@@ -22,6 +22,8 @@ cudaError_t run_stages(const WaveLaunch<T> &L, cudaStream_t s) {
   for (int d = 0; d < L.wb.rays; d++) {
     WaveBufs<T> wbd = L.wb;
     wbd.depth = d;
+    WaveBufs<T> wbo = wbd;   // of the overflow pass
+    wbo.spread = dev::launch_spread(wbd.spread, L.ov_grid * (L.block / 32));
     if (d > 0) {
       WaveBufs<T> wbp = L.wb;
       wbp.depth = d - 1;
@@ -32,12 +34,12 @@ cudaError_t run_stages(const WaveLaunch<T> &L, cudaStream_t s) {
       dev::primary_kernel<T, F, FAST, true><<<L.grid, L.block, 0, s>>>(L.p, L.fd, stage_io(L.io, 0), wbd, L.cams,
                                                                         L.ncams);
       if (L.overflow)
-        dev::primary_kernel<T, F, FAST, true, true><<<L.ov_grid, L.block, 0, s>>>(L.p, L.fd, stage_io(L.ov, 0), wbd,
+        dev::primary_kernel<T, F, FAST, true, true><<<L.ov_grid, L.block, 0, s>>>(L.p, L.fd, stage_io(L.ov, 0), wbo,
                                                                                    L.cams, L.ncams);
     } else {
       dev::primary_kernel<T, F, FAST><<<L.grid, L.block, 0, s>>>(L.p, L.fd, stage_io(L.io, 0), wbd, L.cams, L.ncams);
       if (L.overflow)
-        dev::primary_kernel<T, F, FAST><<<L.ov_grid, L.block, 0, s>>>(L.p, L.fd, stage_io(L.ov, 0), wbd, L.cams,
+        dev::primary_kernel<T, F, FAST><<<L.ov_grid, L.block, 0, s>>>(L.p, L.fd, stage_io(L.ov, 0), wbo, L.cams,
                                                                        L.ncams);
     }
     // with reflections the primary stage's time holds every depth's march, polish and reflection

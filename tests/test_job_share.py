@@ -12,7 +12,7 @@ from mandelbulber_gb300 import _build
 SOURCE = r"""
 #include "job_share.cuh"
 extern "C" void share(unsigned jobs, unsigned spread, unsigned launched, unsigned refill, unsigned *out) {
-  const mbgb::dev::JobShare s = mbgb::dev::job_share(jobs, spread, launched, refill);
+  const mbgb::dev::JobShare s = mbgb::dev::job_share(jobs, mbgb::dev::launch_spread(spread, launched), refill, 0, 0);
   out[0] = s.lanes; out[1] = s.warps; out[2] = s.refill;
 }
 """
@@ -49,4 +49,4 @@ def test_every_job_finds_a_lane_where_there_are_enough(share, spread, launched):
 def test_full_warps_claim_at_the_threshold_that_was_asked_for(share, refill):
     assert share(2_000_000, 2432, 4864, refill) == (32, 62500, refill)
     lanes, _, got = share(19200, 2432, 4864, refill)   # 160x120: eight lanes a warp
-    assert (lanes, got) == (8, min(refill, 2))
+    assert (lanes, got) == (8, max(1, refill // 4))

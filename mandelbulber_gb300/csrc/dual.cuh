@@ -16,17 +16,35 @@ struct Dual {
   T d[K > 0 ? K : 1];   // (K = 0: the value alone, through the same operations)
 };
 
-// FP32 orbits round their values as written here, a product and a sum by themselves or one fused
-// multiply-add, never at the compiler's choice: it contracts each instantiation by itself (FP64 orbits
-// of one and of four tangents differ in the first product of |z|^2, in 34 of 60000 iteration counts
-// near the surface), and a gradient's head takes an orbit as bounded by its value alone (`escapes`).
-__device__ __forceinline__ float v_mul(const float a, const float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float v_add(const float a, const float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float v_norm2(const float x, const float y, const float z) {
-  return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
+// Where an orbit is taken as bounded by its value alone (`escapes`), the orbit with tangents has to take
+// the same values. The compiler contracts each instantiation by itself (FP64 orbits of one and of four
+// tangents differ in 34 of 60000 iteration counts near the surface), so the values of these orbits,
+// FP32 and FP64 of at most one tangent in units that contract, are written as single products, sums
+// and fused multiply-adds.
+template <typename T, int K>
+constexpr bool kPinned = sizeof(T) == 4 || (K <= 1 && !kStrictF64);
+__device__ __forceinline__ float mul_rn(const float a, const float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(const double a, const double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(const float a, const float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(const double a, const double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float fma_rn(const float a, const float b, const float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(const double a, const double b, const double c) { return __fma_rn(a, b, c); }
+template <int K, typename T>
+__device__ __forceinline__ T v_mul(const T a, const T b) {
+  if constexpr (kPinned<T, K>) return mul_rn(a, b);
+  else return a * b;
 }
-__device__ __forceinline__ double v_mul(const double a, const double b) { return a * b; }
-__device__ __forceinline__ double v_add(const double a, const double b) { return a + b; }
+template <int K, typename T>
+__device__ __forceinline__ T v_add(const T a, const T b) {
+  if constexpr (kPinned<T, K>) return add_rn(a, b);
+  else return a + b;
+}
+// x x + y y + z z, the first product fused: y's with YFIRST, else x's
+template <int K, bool YFIRST, typename T>
+__device__ __forceinline__ T v_norm2(const T x, const T y, const T z) {
+  if constexpr (!kPinned<T, K>) return x * x + y * y + z * z;
+  else return fma_rn(z, z, YFIRST ? fma_rn(y, y, mul_rn(x, x)) : fma_rn(x, x, mul_rn(y, y)));
+}
 
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> dconst(const T v) {
@@ -47,7 +65,7 @@ __device__ __forceinline__ Dual<T, K> dseed(const T v, const int k0) {
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> operator+(const Dual<T, K> &a, const Dual<T, K> &b) {
   Dual<T, K> r;
-  r.v = v_add(a.v, b.v);
+  r.v = v_add<K>(a.v, b.v);
 #pragma unroll
   for (int k = 0; k < K; k++) r.d[k] = a.d[k] + b.d[k];
   return r;
@@ -74,14 +92,14 @@ __device__ __forceinline__ Dual<T, K> operator-(const Dual<T, K> &a) {
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> operator+(const Dual<T, K> &a, const T b) {
   Dual<T, K> r = a;
-  r.v = v_add(a.v, b);
+  r.v = v_add<K>(a.v, b);
   return r;
 }
 
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> operator*(const Dual<T, K> &a, const Dual<T, K> &b) {
   Dual<T, K> r;
-  r.v = v_mul(a.v, b.v);
+  r.v = v_mul<K>(a.v, b.v);
 #pragma unroll
   for (int k = 0; k < K; k++) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
   return r;
@@ -90,7 +108,7 @@ __device__ __forceinline__ Dual<T, K> operator*(const Dual<T, K> &a, const Dual<
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> operator*(const Dual<T, K> &a, const T b) {
   Dual<T, K> r;
-  r.v = v_mul(a.v, b);
+  r.v = v_mul<K>(a.v, b);
 #pragma unroll
   for (int k = 0; k < K; k++) r.d[k] = a.d[k] * b;
   return r;
@@ -100,13 +118,13 @@ __device__ __forceinline__ Dual<T, K> operator*(const Dual<T, K> &a, const T b) 
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> dmadd(const Dual<T, K> &a, const Dual<T, K> &b, const Dual<T, K> &c) {
   Dual<T, K> r = a * b + c;
-  if constexpr (sizeof(T) == 4) r.v = __fmaf_rn(a.v, b.v, c.v);
+  if constexpr (kPinned<T, K>) r.v = fma_rn(a.v, b.v, c.v);
   return r;
 }
 template <typename T, int K>
 __device__ __forceinline__ Dual<T, K> dmadd(const Dual<T, K> &a, const Dual<T, K> &b, const T c) {
   Dual<T, K> r = a * b + c;
-  if constexpr (sizeof(T) == 4) r.v = __fmaf_rn(a.v, b.v, c);
+  if constexpr (kPinned<T, K>) r.v = fma_rn(a.v, b.v, c);
   return r;
 }
 
@@ -198,20 +216,22 @@ struct DV3 {
   Dual<T, K> x, y, z;
 };
 
-template <typename T, int K>
+template <bool YFIRST = false, typename T, int K>
 __device__ __forceinline__ Dual<T, K> dlength(const DV3<T, K> &v) {
   if constexpr (sizeof(T) == 4) {
     // FP32: the tangent as (x/r) dx + (y/r) dy + (z/r) dz, without the squares' tangents
     // 2 x dx, which leave FP32's range at an orbit's escape step (x ~ 1e16, dx ~ 1e35)
     Dual<T, K> r;
-    r.v = m_sqrt(v_norm2(v.x.v, v.y.v, v.z.v));
+    r.v = m_sqrt(v_norm2<K, YFIRST>(v.x.v, v.y.v, v.z.v));
     const T inv = r.v > T(0) ? T(1) / r.v : T(0);
     const T ux = v.x.v * inv, uy = v.y.v * inv, uz = v.z.v * inv;
 #pragma unroll
     for (int k = 0; k < K; k++) r.d[k] = ux * v.x.d[k] + uy * v.y.d[k] + uz * v.z.d[k];
     return r;
   } else {
-    return dsqrt(v.x * v.x + v.y * v.y + v.z * v.z);
+    Dual<T, K> q = v.x * v.x + v.y * v.y + v.z * v.z;
+    if constexpr (kPinned<T, K>) q.v = v_norm2<K, YFIRST>(v.x.v, v.y.v, v.z.v);
+    return dsqrt(q);
   }
 }
 
@@ -254,17 +274,17 @@ __device__ __forceinline__ Dual<T, K> de_dual_seeded(const FractalT<T> &f, DV3<T
       if constexpr (sizeof(T) == 4) {
         // r_dz' = A r_dz + 1 with A = r^(p-1) p: d r_dz' / r_dz' = (dA + A q) r_dz / r_dz'
         const D A = rp * p;
-        const T nv = __fmaf_rn(A.v, rdz, 1.0f);
+        const T nv = fma_rn(A.v, rdz, T(1));
         const T ratio = rdz / nv;
 #pragma unroll
         for (int k = 0; k < K; k++) q[k] = (A.d[k] + A.v * q[k]) * ratio;
         rdz = nv;
       } else {
-        r_dz = rp * r_dz * p + T(1);
+        r_dz = dmadd(rp * r_dz, p, T(1));
       }
       rp = rp * r;
       z = {dmadd(cth * cph, rp, c.x), dmadd(cth * sph, rp, c.y), dmadd(sth, rp, c.z)};
-      r = dlength(z);
+      r = dlength<sizeof(T) == 8>(z);
       if (r.v > f.bailout) {
         if constexpr (sizeof(T) == 4) {
           // dist = num / r_dz: d dist = d num / r_dz - dist q
@@ -353,11 +373,16 @@ __device__ __forceinline__ bool escapes(const FractalT<T> &f, const V3<T> P, con
 // reference's binary refinement has put it inside the window (0.99 thr, thr)). Returns
 // false (and leaves t) when the level set is not reached: a grazing ray (F_t >= 0), a
 // flat estimate (orbit not escaping, minN clamp), or no convergence in 16 steps.
+// `bounded`: the FP32 refinement met an orbit that did not escape. Such a hit usually fails here
+// for the same reason after N iterations of the pipe-bound libm orbit, and its chain can bound the
+// stage, so the orbit is first run without tangents, at the same values (kPinned). Of 48 seeds of
+// eight 256x256 frames it takes 12 % off the whole call in four and nothing off the others.
 template <int FORMULA>
 __device__ __forceinline__ bool level_set_hit(const FractalT<double> &f, const V3<double> o, const V3<double> d,
                                               const double k, const double thrConst, double &t, int &iters,
-                                              const double fparam) {
+                                              const double fparam, const bool bounded) {
   double tt = t;
+  if (bounded && !escapes<double, FORMULA>(f, o + d * tt, f.N, fparam)) return false;
   for (int it = 0; it < 16; it++) {
     int L;
     const Dual<double, 1> de = de_along<double, FORMULA>(f, o + d * tt, d, f.N, L, fparam);
@@ -387,13 +412,14 @@ __device__ __forceinline__ bool level_set_hit(const FractalT<double> &f, const V
 template <int FORMULA>
 __device__ __forceinline__ bool level_set_hit_f32(const FractalT<float> &f, const V3<float> o, const V3<float> d,
                                                   const float k, const float thrConst, float &t, int &iters,
-                                                  const float fparam) {
+                                                  const float fparam, bool &bounded) {
   float tt = t;
   const float lenD = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
   for (int it = 0; it < 16; it++) {
     int L;
     const Dual<float, 1> de = de_along<float, FORMULA>(f, o + d * tt, d, f.N, L, fparam);
     const float thr = k > 0.0f ? tt * k : thrConst;
+    if (L == f.N) bounded = it == 0;
     if (L == f.N || L < f.minN || !isfinite(de.v) || !isfinite(de.d[0])) return false;
     const float F = de.v - thr;
     if (fabsf(F) <= 2e-5f * thr) {

@@ -39,7 +39,7 @@ __device__ __forceinline__ Dual<double, 4> de_dual_policy(const ParamsT<T> &p, c
     // A neighbour of the hit inside the set runs all N (1250) iterations and has no derivative; on
     // one lane with four tangents three of them bounded the stage. So the tangents are carried
     // for kGradHead iterations, which nearly every other orbit needs, and a longer one first runs
-    // as the value alone, which rounds as the orbit with tangents does (v_mul, dmadd). Twelve seeds of
+    // as the value alone, which rounds as the orbit with tangents does (kPinned). Twelve seeds of
     // eight 256x256 frames: 4.65 -> 4.22 ms of the whole call on average (1.05 to 1.18 times in
     // ten of them, none slower), identical Jacobians.
     Dual<float, 4> r = de_dual<float, FORMULA>(p.f, q, N < kGradHead ? N : kGradHead, L, fparam);

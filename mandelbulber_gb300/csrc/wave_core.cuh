@@ -1341,6 +1341,7 @@ __global__ void __launch_bounds__(128) level_set_kernel(const __grid_constant__ 
     const FrameCam<T> &c = cams[frame_of_pixel(cams, ncams, gp)];
     const int64_t local = gp - c.pixBase;
     const int x = (int)(local % c.width), y = (int)(local / c.width);
+    bool bounded = false;
     if constexpr (sizeof(T) == 4) {
       // FP32 policy: Newton in FP32 on the march's own ray; FP64 only where that fails
       V3<float> dirf;
@@ -1349,7 +1350,7 @@ __global__ void __launch_bounds__(128) level_set_kernel(const __grid_constant__ 
       const float kf = p.constantDEThreshold ? 0.0f : c.resolution * c.persp / p.quality;
       float tf = wb.scan[gp];
       int lf = wb.iters[gp];
-      if (level_set_hit_f32<FORMULA>(p.f, startf, dirf, kf, p.quality, tf, lf, c.fparam)) {
+      if (level_set_hit_f32<FORMULA>(p.f, startf, dirf, kf, p.quality, tf, lf, c.fparam, bounded)) {
         const float thr = p.constantDEThreshold ? p.quality : tf * kf;
         const V3<float> point = startf + dirf * tf;
         wb.scan[gp] = tf;
@@ -1368,7 +1369,7 @@ __global__ void __launch_bounds__(128) level_set_kernel(const __grid_constant__ 
     const double kd = p.constantDEThreshold ? 0.0 : c.resolution_d * c.persp_d / p.quality_d;
     double t = (double)wb.scan[gp];
     int li = wb.iters[gp];
-    if (level_set_hit<FORMULA>(fd, start, dir, kd, p.quality_d, t, li, c.fparam_d)) {
+    if (level_set_hit<FORMULA>(fd, start, dir, kd, p.quality_d, t, li, c.fparam_d, bounded)) {
       const V3<double> point = start + dir * t;
       const double thr = p.constantDEThreshold ? p.quality_d : t * c.resolution_d * c.persp_d / p.quality_d;
       wb.scan[gp] = (T)t;

@@ -31,7 +31,8 @@ FractalT<T> fractal(const int formula, const int N) {
   return f;
 }
 // counts: [0] points, [1] orbits of more than kGradHead iterations that escape, [2] bounded orbits,
-// differences of [3] de_dual_policy and the plain dual orbit, [4] escapes and the dual orbit
+// differences of [3] de_dual_policy and the plain dual orbit, [4] escapes and the FP32 dual orbit,
+// [5] escapes and the FP64 orbit of the level set
 template <int FORMULA>
 __global__ void compare_kernel(const ParamsT<float> p, const FractalT<double> fd, const double fparam, const int n,
                                const double *points, unsigned long long *count) {
@@ -51,6 +52,10 @@ __global__ void compare_kernel(const ParamsT<float> p, const FractalT<double> fd
     if (M == fd.N) atomicAdd(count + 2, 1ull);
     if (finite && !same) atomicAdd(count + 3, 1ull);
     if (escapes<float, FORMULA>(p.f, q, fd.N, (float)fparam) != (M < fd.N)) atomicAdd(count + 4, 1ull);
+    if (i % 8 == 0) {
+      de_along<double, FORMULA>(fd, P, V3<double>{0.3, 0.9, -0.2}, fd.N, M, fparam);
+      if (escapes<double, FORMULA>(fd, P, fd.N, fparam) != (M < fd.N)) atomicAdd(count + 5, 1ull);
+    }
   }
 }
 }
@@ -86,10 +91,10 @@ def test_value_only_orbits_are_the_dual_orbits(lib, formula, N, fparam):
         p = rng.uniform(-6.0, 6.0, (n, 3))
         p[: n // 2] *= 0.2
     points = torch.tensor(p, device="cuda")
-    count = torch.zeros(5, dtype=torch.int64, device="cuda")
+    count = torch.zeros(6, dtype=torch.int64, device="cuda")
     torch.cuda.synchronize()
     assert lib.compare(formula, N, ctypes.c_double(fparam), n, ctypes.c_void_p(points.data_ptr()),
                        ctypes.c_void_p(count.data_ptr())) == 0
-    total, late, bounded, policy, escapes = count.tolist()
+    total, late, bounded, policy, fp32, fp64 = count.tolist()
     assert total == n and bounded > 0 and (formula == 8 or late > 100)
-    assert (policy, escapes) == (0, 0)
+    assert (policy, fp32, fp64) == (0, 0, 0)

@@ -18,19 +18,20 @@ __host__ __device__ __forceinline__ unsigned int at_least_one(const unsigned int
 // `refill`: idle lanes before a warp claims again, refill_min of 32 in proportion to its lanes.
 struct JobShare {
   unsigned int lanes, warps, refill;
-  bool idle;   // this lane takes none (the kernels set it)
+  bool idle;   // this lane takes none
 };
 
-// A stage with fewer jobs than lanes hands each warp only as many as let `spread` warps take part,
-// and only the first warps take any (blocks start one per SM, so those spread evenly over the SMs and
-// their sub-partitions).
+// The share of lane `lane` of warp `warp`. A stage with fewer jobs than lanes hands each warp only as
+// many as let `spread` warps take part, and only the first warps take any (blocks start one per SM, so
+// those spread evenly over the SMs and their sub-partitions).
 __host__ __device__ __forceinline__ JobShare job_share(const unsigned int jobs, const unsigned int spread,
-                                                       const unsigned int refill_min) {
+                                                       const unsigned int refill_min, const unsigned int warp,
+                                                       const unsigned int lane) {
   JobShare s;
   s.lanes = jobs >= 32u * spread ? 32u : at_least_one((jobs + spread - 1) / spread);
   s.warps = (jobs + s.lanes - 1) / s.lanes;
   s.refill = at_least_one(s.lanes * refill_min / 32u);
-  s.idle = false;
+  s.idle = lane >= s.lanes || warp >= s.warps;
   return s;
 }
 

@@ -356,10 +356,8 @@ __device__ __forceinline__ unsigned int claim_jobs(unsigned int *counter, const 
 // This lane's share of a stage's `jobs`.
 template <typename T>
 __device__ __forceinline__ JobShare job_share(const WaveBufs<T> &wb, const unsigned int jobs) {
-  JobShare s = job_share(jobs, (unsigned int)wb.spread, (unsigned int)wb.refill_min);
-  const unsigned int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  s.idle = (threadIdx.x & 31u) >= s.lanes || warp >= s.warps;
-  return s;
+  return job_share(jobs, (unsigned int)wb.spread, (unsigned int)wb.refill_min,
+                   blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31u);
 }
 
 // One pooled step record: dist, thr, step in a 16-byte (float) or 32-byte (double) slot.
@@ -1185,8 +1183,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const __grid_constant__ Par
   const double search_limit = 1.0 - 0.01 * p.quality_d;
   const unsigned int lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
   const unsigned int warps = gridDim.x * wpb;
-  // (the grid is 8 blocks per SM: an eighth of its warps is one per sub-partition with 128 threads
-  // a block, every other with 64)
+  // (the grid is 8 blocks per SM: an eighth of its warps is one per sub-partition)
   const unsigned int spread = max(1u, warps / 8u);
   const unsigned int lanes = nh >= spread * 32u ? 32u : (nh + spread - 1) / spread;
   for (unsigned int w = blockIdx.x * wpb + (threadIdx.x >> 5); w * lanes < nh; w += warps) {

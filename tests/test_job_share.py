@@ -12,7 +12,7 @@ from mandelbulber_gb300 import _build
 SOURCE = r"""
 #include "job_share.cuh"
 extern "C" void share(unsigned jobs, unsigned spread, unsigned launched, unsigned refill, unsigned *out) {
-  const mbgb::dev::JobShare s = mbgb::dev::job_share(jobs, mbgb::dev::launch_spread(spread, launched), refill);
+  const mbgb::dev::JobShare s = mbgb::dev::job_share(jobs, mbgb::dev::launch_spread(spread, launched), refill, 0, 0);
   out[0] = s.lanes; out[1] = s.warps; out[2] = s.refill;
 }
 """

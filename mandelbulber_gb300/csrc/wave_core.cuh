@@ -2904,7 +2904,7 @@ __device__ __forceinline__ uint16_t u16_of(const float v) {
   const uint32_t b = __float_as_uint(v), e = (b >> 23) & 0xffu;
   if (e < 110u || !(fabsf(v) <= 32768.5f)) return 0;
   const uint64_t prod = (uint64_t)((b & 0x7fffffu) | 0x800000u) * 65535u;
-  const uint32_t q = (uint32_t)(prod >> (150u - e));   // (e <= 142)
+  const uint32_t q = e <= 150u ? (uint32_t)(prod >> (150u - e)) : (uint32_t)(prod << (e - 150u));
   return (uint16_t)(v < 0.0f ? 0u - q : q);
 }
 __device__ __forceinline__ uint8_t u8_of(const double v) { return to_u8_x86(v); }

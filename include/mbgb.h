@@ -234,7 +234,8 @@ typedef struct mbgb_opts {
                                 * hits whose FP32 bisection stopped early within 1e-4 of a window edge */
   int32_t tile_w, tile_h;      /* wavefront: pixel tile of a warp's first 32 primary rays (tile_w * tile_h
                                 * = 32); 0,0 = autotuned or 8 x 4 */
-  int32_t refill_min;          /* wavefront: idle lanes of a warp before it claims new rays; 0 = tuned or 8 */
+  int32_t refill_min;          /* wavefront: idle lanes of a warp before it claims new rays (in proportion where
+                                * a small stage fills only some lanes of its warps); 0 = tuned or 8 */
   int32_t autotune;            /* 1: tile shape, threads per CTA, CTAs per SM and refill_min that are 0
                                 * come from mbgb_autotune, run once per scene class and context */
   int32_t use_graph;           /* 1: the launches are captured once in a CUDA graph and replayed while

@@ -273,10 +273,10 @@ static int distance_kernel_formula(const mbgb_scene &s) {
 }
 
 // The lean FP32 Mandelbox orbit applies: formula 8 without rotations, offset, pre-folds,
-// julia or primitive objects, fold value = 2 x fold limit, and min radius <= fixed radius in
-// magnitude too, since the fold takes their squares (so that the sphere fold is a clamp). The limit box, interior mode and the iteration threshold
-// only test the point before the orbit or post-process its result (limit_box, distance_post),
-// which every lean path applies.
+// julia or primitive objects, fold value = 2 x fold limit, and min radius <= fixed radius, in
+// magnitude too, since the fold takes their squares (so that the sphere fold is a clamp). The limit
+// box, interior mode and the iteration threshold only test the point before the orbit or
+// post-process its result (limit_box, distance_post), which every lean path applies.
 static bool fast_mandelbox(const mbgb_scene &s) {
   return s.formula == MBGB_FORMULA_TGLAD && !s.mboxRotationsEnabled && s.mboxMainRotZero && !s.juliaMode &&
          !s.tgladFoldingMode && !s.sphericalFoldingMode && !s.ifsFoldingMode && !uses_primitives(s) &&

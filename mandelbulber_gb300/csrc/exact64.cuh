@@ -180,7 +180,7 @@ __host__ __device__ __forceinline__ double mul_exact(const double a, const doubl
 __device__ __forceinline__ bool int_range(const double a) {
   return ((uint32_t)(f64_bits(a) >> 52) & 0x7ffu) - 600u <= 800u;
 }
-// a * b with b in [2^-300, 2^300]
+// a * b with b in [2^-400, 2^400]
 __device__ __forceinline__ double mul_int(const double a, const double b) {
   return int_range(a) ? mul_exact(a, b) : __dmul_rn(a, b);
 }

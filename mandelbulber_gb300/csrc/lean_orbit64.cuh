@@ -1,5 +1,5 @@
 // The Mandelbox orbit (formula 8, normal mode) of the FP64 policy, with the reference's
-// results bit for bit at a third of the FP64 instructions of compute<double, 8, 0>.
+// results bit for bit at an eighth of the FP64 instructions of compute<double, 8, 0>.
 //
 // What bounds it: GB300's FP64 pipe, 20 SM cycles per warp instruction (exact64.cuh). The
 // generic iteration (tglad_step) issues 61 of them; here the usual iteration issues 8, beside
@@ -9,8 +9,9 @@
 //     monotonically), so each is q against a bound that the host derives exactly
 //     (FractalT::boxQIn, boxQMid, boxQBail), and a comparison of positive doubles is one of
 //     their bits: integer instructions. |x| > limit likewise.
-//   * In the shell, r * r and fR2 / (r * r) come from integer multiplies (sqrt_squared,
-//     div_exact: 88 SM cycles in otherwise empty issue slots against 260 on the pipe).
+//   * In the shell, r * r and fR2 / (r * r) come from integer multiplies (sqrt_squared and
+//     div_exact, 33 SM cycles each in otherwise empty issue slots; on the pipe the root takes 156, its
+//     square 20 and the quotient 90).
 //   * With a scale and an inner fold factor that are powers of two (the usual 2 and 4) the
 //     products are exact, so z * k * scale + c is one fused multiply-add. Other scales take the
 //     two roundings.
@@ -20,7 +21,7 @@
 //     squares too: 25.3 -> 23.2 ms for a frame, whose stages have fewer active lanes and free issue
 //     slots, but 1.07 -> 1.11 ms for that loop of full warps, which keeps them (FULL).
 // Measured: 2,000,003 distances (N 15) 3.92 ms generic, 1.44 ms with the pipe for fold and
-// products, 0.96 ms as it stands; a 481x271 Mandelbox frame 92.9 -> 28.0 ms.
+// products, 0.96 ms as it stands; a 481x271 Mandelbox frame 89.8 -> 22.6 ms.
 // Not kept: leaving out the bailout test of the first five iterations, which a start point near
 // the box cannot fail, made the loop slower in every form tried (1.17 -> 1.29 to 1.35 ms).
 #pragma once

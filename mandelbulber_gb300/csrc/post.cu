@@ -192,7 +192,8 @@ __global__ void ssao_kernel(const float *__restrict__ zbuf, const uint16_t *__re
   }
 }
 
-// Pairs of floats (value hi + lo, about 46 bits) for the horizon angles.
+// Pairs of floats (value hi + lo, about 46 bits) for the horizon angles: Knuth's and Dekker's
+// error-free sums, products with the residual of a fused multiply-add.
 struct F2 {
   float h, l;
 };
@@ -390,7 +391,7 @@ __device__ __forceinline__ bool ssao_sample(const SsaoArgs &g, const SsaoSample 
 //     instruction of the FP64 pipe costs its 20 cycles even with no lane active: the pass has none.)
 // What bounds it now is the first pass's issue rate, about 40 instructions a sample.
 // 1920x1080, quality 20, with the 16-bit step: every slope in double 70.6 ms, the steepest only
-// in double 5.65 ms, as it stands 2.41 ms.
+// in double 5.65 ms, as it stands 2.30 ms.
 __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ SsaoArgs g) {
   const int64_t n = (int64_t)g.width * g.height;
   const double w = (double)g.width, h = (double)g.height, aspect = w / h;
@@ -500,9 +501,9 @@ __global__ void __launch_bounds__(128) ssao_flat_kernel(const __grid_constant__ 
 // values of ssao_kernel<double> bit for bit): a lane takes a direction (every 32nd of more than 32),
 // and the directions' terms are summed in the reference's order. A warp holds as many pixels as
 // leave a lane to each direction: with one each, a frame whose depths all lie below the FP32 forms'
-// range (a camera a millionth from the surface) took longer than ssao_kernel<double>, 1024x768 at
-// quality 4 / 6 / 10 / 20 6.7 / 8.5 / 12.1 / 21.8
-// against 1.33 / 2.84 / 7.7 / 30.4 ms, as it stands 0.88 / 2.13 / 5.9 / 20.8.
+// range (a camera a millionth from the surface) took longer than ssao_kernel<double>: 1024x768 at
+// quality 4 / 6 / 10 / 20 6.7 / 8.5 / 12.1 / 21.8 ms against 1.33 / 2.84 / 7.7 / 30.4, as it stands
+// 0.88 / 2.13 / 5.9 / 20.8.
 __global__ void __launch_bounds__(128) ssao_exact_kernel(const __grid_constant__ SsaoArgs g) {
   using mbgb::dev::div_int;
   using mbgb::dev::sqrt_int;

@@ -1183,7 +1183,8 @@ __global__ void __launch_bounds__(128) polish_kernel(const __grid_constant__ Par
   const double search_limit = 1.0 - 0.01 * p.quality_d;
   const unsigned int lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
   const unsigned int warps = gridDim.x * wpb;
-  // (the grid is 8 blocks per SM: an eighth of its warps is one per sub-partition)
+  // (the grid is 8 blocks per SM: an eighth of its warps is one per sub-partition with 128 threads
+  // a block, every other with 64)
   const unsigned int spread = max(1u, warps / 8u);
   const unsigned int lanes = nh >= spread * 32u ? 32u : (nh + spread - 1) / spread;
   for (unsigned int w = blockIdx.x * wpb + (threadIdx.x >> 5); w * lanes < nh; w += warps) {
@@ -2904,6 +2905,8 @@ __device__ __forceinline__ uint16_t u16_of(const float v) {
   const uint32_t b = __float_as_uint(v), e = (b >> 23) & 0xffu;
   if (e < 110u || !(fabsf(v) <= 32768.5f)) return 0;
   const uint64_t prod = (uint64_t)((b & 0x7fffffu) | 0x800000u) * 65535u;
+  // (e is at most 142 here, so the left shift is never taken; without its branch the effects variant's
+  // composition ran 2.20 ms instead of 2.14 at the same registers, 480x270 Menger sponge)
   const uint32_t q = e <= 150u ? (uint32_t)(prod >> (150u - e)) : (uint32_t)(prod << (e - 150u));
   return (uint16_t)(v < 0.0f ? 0u - q : q);
 }
